@@ -50,10 +50,13 @@
 #include <vector>
 
 #include "acfdtd_b200.h"
+#include "acfdtd_device.cuh"
+#include "acfdtd_resident.cuh"
+
+using namespace acf;
 
 namespace {
 
-constexpr int kVec = 4;            // elements per thread along z
 constexpr int kRowAlign = 8;       // row pitch granularity, elements
 constexpr int kEnergyTerms = 7;
 
@@ -74,155 +77,6 @@ int fail(int code, const char *fmt, ...) {
             return fail(ACF_ERR_CUDA, "%s failed: %s (%s:%d)", #call,                      \
                         cudaGetErrorString(err__), __FILE__, __LINE__);                    \
     } while (0)
-
-// ------------------------------------------------------------------------------------------
-// Vector access: 4 consecutive elements, one 16-byte access for float, two for double.
-
-template <typename T>
-struct Vec4;
-
-template <>
-struct Vec4<float> {
-    __device__ __forceinline__ static void load(const float *__restrict__ a, float v[4]) {
-        const float4 t = *reinterpret_cast<const float4 *>(a);
-        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    }
-    __device__ __forceinline__ static void store(float *__restrict__ a, const float v[4]) {
-        *reinterpret_cast<float4 *>(a) = make_float4(v[0], v[1], v[2], v[3]);
-    }
-    // Read-only path: only for arrays no thread writes during the kernel.
-    __device__ __forceinline__ static void ldg(const float *__restrict__ a, float v[4]) {
-        const float4 t = __ldg(reinterpret_cast<const float4 *>(a));
-        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    }
-    // Streaming (evict-first) load: data read once, such as the adjoint's history.
-    __device__ __forceinline__ static void ldcs(const float *a, float v[4]) {
-        const float4 t = __ldcs(reinterpret_cast<const float4 *>(a));
-        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    }
-};
-
-template <>
-struct Vec4<double> {
-    __device__ __forceinline__ static void load(const double *__restrict__ a, double v[4]) {
-        const double2 t0 = *reinterpret_cast<const double2 *>(a);
-        const double2 t1 = *reinterpret_cast<const double2 *>(a + 2);
-        v[0] = t0.x; v[1] = t0.y; v[2] = t1.x; v[3] = t1.y;
-    }
-    __device__ __forceinline__ static void store(double *__restrict__ a, const double v[4]) {
-        *reinterpret_cast<double2 *>(a) = make_double2(v[0], v[1]);
-        *reinterpret_cast<double2 *>(a + 2) = make_double2(v[2], v[3]);
-    }
-    __device__ __forceinline__ static void ldg(const double *__restrict__ a, double v[4]) {
-        const double2 t0 = __ldg(reinterpret_cast<const double2 *>(a));
-        const double2 t1 = __ldg(reinterpret_cast<const double2 *>(a + 2));
-        v[0] = t0.x; v[1] = t0.y; v[2] = t1.x; v[3] = t1.y;
-    }
-    __device__ __forceinline__ static void ldcs(const double *a, double v[4]) {
-        const double2 t0 = __ldcs(reinterpret_cast<const double2 *>(a));
-        const double2 t1 = __ldcs(reinterpret_cast<const double2 *>(a + 2));
-        v[0] = t0.x; v[1] = t0.y; v[2] = t1.x; v[3] = t1.y;
-    }
-};
-
-// Streaming (evict-first) stores of 4 elements, for data written once and read once much later
-// -- the adjoint's D/psi history -- so that it does not push the state out of L2.
-__device__ __forceinline__ void store_streaming(float *a, const float v[4]) {
-    __stcs(reinterpret_cast<float4 *>(a), make_float4(v[0], v[1], v[2], v[3]));
-}
-__device__ __forceinline__ void store_streaming(double *a, const double v[4]) {
-    __stcs(reinterpret_cast<double2 *>(a), make_double2(v[0], v[1]));
-    __stcs(reinterpret_cast<double2 *>(a + 2), make_double2(v[2], v[3]));
-}
-
-// Ask L2 for the line holding `a` ahead of its load: the request holds no register and no
-// shared memory, so a marching thread can have its next plane on the way from DRAM while it
-// computes the current one. Only addresses the thread will load later are passed.
-template <typename T>
-__device__ __forceinline__ void prefetch_l2(const T *a) {
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
-}
-
-// Bits of a handle's device status word.
-constexpr int32_t kStatusWaitTimeout = 1;   // a staged sweep gave up waiting for its copies
-constexpr int32_t kStatusNonFinite = 2;     // a sweep produced a NaN or infinite pressure
-
-__device__ __forceinline__ unsigned lane_id() {
-    unsigned lane;
-    asm("mov.u32 %0, %%laneid;" : "=r"(lane));
-    return lane;
-}
-
-// Non-finite detector: acc = fma(x, 0, acc) is acc + 0 for every finite x (one rounding, exact)
-// and NaN once any x was NaN or infinite; NaN then stays. One fused instruction per value.
-template <typename T>
-__device__ __forceinline__ T finite_acc(T acc, T x) {
-    if constexpr (sizeof(T) == 4) return __fmaf_rn(x, 0.0f, acc);
-    else return __fma_rn(x, 0.0, acc);
-}
-
-// Raise kStatusNonFinite once per warp whose threads saw a non-finite value.
-__device__ __forceinline__ void report_nonfinite(int32_t *status, bool bad) {
-    const unsigned mask = __ballot_sync(__activemask(), bad);
-    if (bad && status != nullptr && lane_id() == (unsigned)(__ffs(mask) - 1))
-        atomicOr(status, kStatusNonFinite);
-}
-
-// ------------------------------------------------------------------------------------------
-// What the sweeps read about one room. Plain data, identical on host and device.
-
-template <typename T>
-struct Room {
-    int32_t nx, ny, nz, nchunks;
-    int32_t prefetch;              // 1: marching threads ask L2 for their next plane ahead
-    int32_t reserved;
-    // A slab of a room cut along x: the single-room pressure sweep updates the planes
-    // [own_lo, own_hi) only, and also stores p of planes own_lo and own_hi - 1 into the
-    // neighbours' ghost planes (null: no neighbour on that side; a peer address when the
-    // neighbour lives on another GPU). A whole room: [0, nx), no ghosts.
-    int32_t own_lo, own_hi;
-    T *ghost_lo, *ghost_hi;
-    int64_t pz, plane, field;      // row pitch, plane pitch, elements per field
-    T *p, *vx, *vy, *vz, *psi;     // psi: n_relax fields back to back
-    T cv, cp, cs, relax_scale;
-    T decay[ACF_MAX_RELAXATION], mean[ACF_MAX_RELAXATION], gain[ACF_MAX_RELAXATION];
-    const T *cell[3];              // layer profiles at cell centres
-    const T *face[3];              // layer profiles at faces
-    const T *shell[6];             // wall pairs (1/(1+a), a/(1+a)) per face cell
-    int32_t n_src;
-    int32_t n_rec;
-    const int64_t *src_off;        // padded offsets
-    const int64_t *src_len;
-    const T *src_sig;
-    int64_t src_stride;
-    const int64_t *rec_off;        // padded offsets
-    const int64_t *rec_start;      // first absolute step recorded
-    const int64_t *src_col;        // in-plane offsets (padded offset mod plane): j * pz + k
-    const int64_t *rec_col;
-    T *rec;
-    int64_t rec_stride, rec_origin;
-    // Status word of the handle (device memory): the sweeps that write p set kStatusNonFinite
-    // in it when a pressure they produced is NaN or infinite. Null: not checked.
-    int32_t *status;
-};
-
-// Forward history kept for the adjoint: per step, p^n and p-tilde^n -- pressure before the step
-// and before the wall closed form -- on every boundary cell (two blocks of shell_total values,
-// first every p^n, then every p-tilde^n), and, for a
-// segment of steps, the divergence D^n and the relaxation states psi^n before their update.
-// Boundary cells are indexed as in the wall shells: the first face of FACES order a cell lies
-// on, then row-major over that face's two other axes; face f starts at face_off[f].
-template <typename T>
-struct History {
-    T *shell;                      // steps x 2 x shell_total values, or null
-    int64_t shell_total, shell_step0, shell_steps;
-    int64_t face_off[6];
-    T *fields;                     // slots x (1 + n_relax) fields (padded geometry), or null;
-                                   // step n uses slot (n - fields_step0) mod fields_slots
-    int64_t fields_step0;
-    int32_t fields_slots;
-    int32_t reserved;
-};
 
 template <typename T>
 struct StepParams {
@@ -362,169 +216,6 @@ __device__ __forceinline__ void velocity_column(const Room<T> &s, int i_begin, i
 // ------------------------------------------------------------------------------------------
 // (b) pressure, one column. The velocities are read-only here; p and psi are read and written
 // by their owning thread only. vx of the upper face is carried into the next plane's lower face.
-
-// First face (FACES order) that cell (i, j, k) lies on, and its index within that face's
-// row-major (b, c) array; -1 for interior cells.
-template <typename T>
-__device__ __forceinline__ int shell_face(const Room<T> &s, int i, int j, int k, int64_t &idx) {
-    if (i == 0) { idx = (int64_t)j * s.nz + k; return 0; }
-    if (i == s.nx - 1) { idx = (int64_t)j * s.nz + k; return 1; }
-    if (j == 0) { idx = (int64_t)i * s.nz + k; return 2; }
-    if (j == s.ny - 1) { idx = (int64_t)i * s.nz + k; return 3; }
-    if (k == 0) { idx = (int64_t)i * s.ny + j; return 4; }
-    if (k == s.nz - 1) { idx = (int64_t)i * s.ny + j; return 5; }
-    return -1;
-}
-
-template <typename T>
-__device__ __forceinline__ bool wall_pair(const Room<T> &s, int i, int j, int k, T &fu, T &fp) {
-    int64_t idx;
-    const int f = shell_face(s, i, j, k, idx);
-    if (f < 0) return false;
-    const T *entry = s.shell[f] + 2 * idx;
-    fu = __ldg(entry);
-    fp = __ldg(entry + 1);
-    return fp != T(0) || fu != T(1);
-}
-
-// The wall closed form for the cells of one column chunk at plane i: on an x-face plane or a
-// y-face row (both uniform across a warp) every cell is tested; elsewhere only the chunk's
-// k = 0 and k = nz - 1 cells can lie on a face -- a z face, the first in FACES order for them --
-// so the thread reads just those pairs instead of searching four cells. `apply(e, fu, fp)` is
-// called for each cell e (< real) with an absorbing pair.
-template <typename T, typename Apply>
-__device__ __forceinline__ void column_walls(const Room<T> &s, int i, int j, int k0, int real,
-                                             Apply apply) {
-    if (i == 0 || i == s.nx - 1 || j == 0 || j == s.ny - 1) {
-#pragma unroll
-        for (int e = 0; e < kVec; e++) {
-            T fu, fp;
-            if (e < real && wall_pair(s, i, j, k0 + e, fu, fp)) apply(e, fu, fp);
-        }
-        return;
-    }
-    const bool bottom = k0 == 0, top_chunk = k0 + kVec >= s.nz;
-    if (!bottom && !top_chunk) return;
-    const int64_t at = 2 * ((int64_t)i * s.ny + j);
-    if (bottom) {
-        const T fu = __ldg(s.shell[4] + at), fp = __ldg(s.shell[4] + at + 1);
-        if (fp != T(0) || fu != T(1)) apply(0, fu, fp);
-    }
-    const int top = s.nz - 1 - k0;
-    if (top_chunk && (top > 0 || k0 > 0)) {     // k = nz - 1 is not also k = 0
-        const T fu = __ldg(s.shell[5] + at), fp = __ldg(s.shell[5] + at + 1);
-        if (fp != T(0) || fu != T(1)) apply(top, fu, fp);
-    }
-}
-
-// Sources (bit q) and receivers (bit n_src + r) that lie in one (row j, chunk at k0) column,
-// found once per column so that the march visits them only at their own plane instead of
-// scanning every point at every plane. Beyond 32 points `all` is set and every point is
-// scanned, as before.
-template <typename T>
-__device__ __forceinline__ uint32_t column_points(const Room<T> &s, int j, int k0, bool &all,
-                                                 int width = kVec) {
-    const int total = s.n_src + s.n_rec;
-    all = total > 32;
-    uint32_t mask = 0;
-    if (all) return 0;
-    const int64_t first = (int64_t)j * s.pz + k0;
-    for (int q = 0; q < total; q++) {
-        const int64_t col = q < s.n_src ? s.src_col[q] : s.rec_col[q - s.n_src];
-        if (col >= first && col < first + width) mask |= 1u << q;
-    }
-    return mask;
-}
-
-__device__ __forceinline__ uint32_t source_bits(uint32_t mask, int n_src) {
-    return n_src >= 32 ? mask : mask & ((1u << n_src) - 1u);
-}
-
-__device__ __forceinline__ uint32_t receiver_bits(uint32_t mask, int n_src) {
-    return n_src >= 32 ? 0u : mask >> n_src;
-}
-
-// Sources of the column's cell at `base`, after damping, in the order they were added
-// (scheme.py:293,360-363).
-template <typename T>
-__device__ __forceinline__ void add_sources(const Room<T> &s, uint32_t mask, bool all, int64_t base,
-                                            int k0, int64_t step, T Pn[kVec]) {
-    uint32_t m = all ? 0u : source_bits(mask, s.n_src);
-    for (int q = all ? 0 : -1; all ? q < s.n_src : m != 0; q++) {
-        if (!all) {
-            q = __ffs(m) - 1;
-            m &= m - 1;
-        }
-        const int64_t d = s.src_off[q] - base;
-        if (d >= 0 && d < kVec && k0 + d < s.nz && step < s.src_len[q]) {
-#pragma unroll
-            for (int e = 0; e < kVec; e++)
-                if (e == d) Pn[e] = Pn[e] + s.cs * s.src_sig[q * s.src_stride + step];
-        }
-    }
-}
-
-// Receivers of the column read the finished pressure (scheme.py:294-296).
-template <typename T>
-__device__ __forceinline__ void record_receivers(const Room<T> &s, uint32_t mask, bool all,
-                                                 int64_t base, int64_t step, const T Pn[kVec]) {
-    uint32_t m = all ? 0u : receiver_bits(mask, s.n_src);
-    for (int r = all ? 0 : -1; all ? r < s.n_rec : m != 0; r++) {
-        if (!all) {
-            r = __ffs(m) - 1;
-            m &= m - 1;
-        }
-        const int64_t d = s.rec_off[r] - base;
-        if (d >= 0 && d < kVec && step >= s.rec_start[r]) {
-            T v = Pn[0];
-#pragma unroll
-            for (int e = 1; e < kVec; e++)
-                if (e == d) v = Pn[e];
-            s.rec[r * s.rec_stride + (step - s.rec_origin)] = v;
-        }
-    }
-}
-
-// Boundary history of one step for the wall gradients: p^n and p before the wall closed form,
-// on every boundary cell, in two blocks of shell_total values per step (first p, then the other)
-// indexed as the wall shells are -- each cell on the first face of FACES order it lies on, then
-// row-major over that face's two other axes. A column on an x-face plane or a y-face row owns
-// contiguous entries for its whole chunk; elsewhere only its k = 0 and k = nz - 1 cells are on a
-// (z) face.
-template <typename T>
-__device__ __forceinline__ void record_shell(const Room<T> &s, const History<T> &hist, int i, int j,
-                                             int k0, int64_t step, const T P[kVec], const T PT[kVec]) {
-    const int64_t slot = step - hist.shell_step0;
-    if (slot < 0 || slot >= hist.shell_steps) return;
-    T *hp = hist.shell + slot * 2 * hist.shell_total;
-    T *ht = hp + hist.shell_total;
-    if (i == 0 || i == s.nx - 1 || j == 0 || j == s.ny - 1) {
-        const bool x_face = i == 0 || i == s.nx - 1;
-        const int f = x_face ? (i == 0 ? 0 : 1) : (j == 0 ? 2 : 3);
-        const int64_t at = hist.face_off[f] + (x_face ? (int64_t)j : (int64_t)i) * s.nz + k0;
-#pragma unroll
-        for (int e = 0; e < kVec; e++)
-            if (k0 + e < s.nz) {
-                hp[at + e] = P[e];
-                ht[at + e] = PT[e];
-            }
-        return;
-    }
-    const int64_t at = (int64_t)i * s.ny + j;
-    if (k0 == 0) {
-        hp[hist.face_off[4] + at] = P[0];
-        ht[hist.face_off[4] + at] = PT[0];
-    }
-    const int top = s.nz - 1 - k0;   // element of k = nz - 1, unless that cell is also k = 0
-    if (s.nz > 1 && top >= 0 && top < kVec) {
-#pragma unroll
-        for (int e = 0; e < kVec; e++)
-            if (e == top) {
-                hp[hist.face_off[5] + at] = P[e];
-                ht[hist.face_off[5] + at] = PT[e];
-            }
-    }
-}
 
 template <typename T, bool LAYER, bool WALLS, int NR, bool REC = false>
 __device__ __forceinline__ void pressure_column(const Room<T> &s, int i_begin, int i_end, int j,
@@ -887,8 +578,6 @@ __global__ void __launch_bounds__(256, ACF_FUSED_MIN_BLOCKS(T, LAYER, NR)) fused
 constexpr int kStagedBarrierBytes = 128;       // full[8] then empty[8] mbarriers
 constexpr int kStagedMaxStages = 8;
 constexpr int kStagedMaxConsumers = 256;      // compute threads per CTA; one producer warp more
-constexpr uint64_t kWaitLimitNs = 2000000000ull;
-constexpr int kWaitLimitIterations = 1 << 21;
 
 template <typename T>
 struct StagedParams {
@@ -909,26 +598,6 @@ struct StagedParams {
 
 // Slots of StagedParams::pairs; the Neg slots hold the negated coefficient.
 enum { kPairCv = 0, kPairCp = 1, kPairNegRelaxScale = 2, kPairGain = 3, kPairNegDecay = 7, kPairNegMean = 11 };
-
-// Packed single precision (sm_100 f32x2), each lane rounded exactly as the scalar operation it
-// replaces. a +- b is the fused a + (+-1) b: the product by +-1 is exact, so the one rounding is
-// that of a +- b. The code generator was measured to fuse a packed multiply into a packed add
-// that consumes it -- one rounding where the reference has two -- even with contraction
-// disabled, and even through a + 1 * b; it was not measured to do so through a - b. So every
-// "plus a product" below is written as "minus the product by the negated coefficient", which
-// rounds identically (negation is exact and rounding is symmetric in sign), and add2 only ever
-// adds values that are not products.
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    return __ffma2_rn(b, make_float2(1.0f, 1.0f), a);
-}
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-    return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a);
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 dup2(float x) { return make_float2(x, x); }
-__device__ __forceinline__ float2 damp2(float2 v, float2 fa, float2 fb, float2 fc) {
-    return mul2(mul2(mul2(v, fa), fb), fc);
-}
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -959,12 +628,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
         : "r"(smem_u32(bar)), "r"(parity), "r"(1000u)
         : "memory");
     return done != 0;
-}
-
-__device__ __forceinline__ uint64_t global_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
 }
 
 // Bounded wait: false when the phase completed neither within `limit_ns` (kWaitLimitNs unless
@@ -1515,8 +1178,6 @@ struct LeanParams {
     float2 pairs[16];      // the slots of StagedParams::pairs
 };
 
-__device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
-__device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
 
 // The per-column constants of a lean column: its place, its edges, its sources and receivers and
 // the y and z layer factors of its cells and faces.
@@ -3859,6 +3520,13 @@ struct acf_batch {
     size_t pair_counters = 0;
     float *psi2 = nullptr;
 
+    // Rooms held on chip (acfdtd_resident.cuh): how the room is cut, found at the first run that
+    // asks (resident_state 0 until then; 1 usable, -1 not), the neighbours' inboxes and tags.
+    int resident_state = 0;
+    ResidentPlan resident;
+    void *resident_mailbox = nullptr;
+    uint32_t *resident_epoch = nullptr;
+
     // CUDA graphs of the adjoint path: forward record, recompute, adjoint steps
     struct Graph {
         cudaGraphExec_t exec = nullptr;
@@ -4483,8 +4151,71 @@ void launch_step(acf_batch *b, int32_t local, cudaStream_t st, cudaEvent_t *even
     if (events) cudaEventRecord(events[2], st);
 }
 
+// Steps from which a run takes the resident sweep, and the most of them in one launch.
+constexpr int64_t kResidentMinSteps = 8, kResidentMaxSteps = 2048;
+
+// Whether this run's steps go through the resident sweep: one room on the two-sweep or the fused
+// scheme, run in several steps per host call (a solver set to launch step by step, or timing its
+// sweeps, gets the sweeps it asked for), with a plan that fits the device and its inboxes in
+// place. They are allocated here, once per handle; where that fails, and inside a stream capture,
+// the sweeps are used as they are without it. Eight steps: loading and storing the state costs
+// as much as two steps of the sweeps.
+template <typename T>
+bool resident_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
+    if (b->resident_state < 0 || n_steps < kResidentMinSteps || b->rooms.size() != 1 || b->profiling ||
+        b->graph_steps == 0 || (b->scheme != ACF_SCHEME_TWO_SWEEPS && b->scheme != ACF_SCHEME_FUSED) ||
+        (b->scheme == ACF_SCHEME_FUSED && b->time_block != 1))
+        return false;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    if (b->resident_state > 0) return true;
+    b->resident_state = -1;
+    const RoomHost &h = b->rooms[0];
+    b->resident = resident_plan<T>(h.nx, h.ny, h.nz, h.n_relax, h.has_layer, b->sms, (size_t)b->smem_per_block);
+    if (b->resident.planes == 0) return false;
+    if (cudaMalloc(&b->resident_mailbox, b->resident.mailbox_bytes) != cudaSuccess ||
+        cudaMalloc(&b->resident_epoch, 2 * sizeof(uint32_t)) != cudaSuccess ||
+        cudaMemsetAsync(b->resident_mailbox, 0, b->resident.mailbox_bytes, st) != cudaSuccess ||
+        cudaMemsetAsync(b->resident_epoch, 0, 2 * sizeof(uint32_t), st) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    b->resident_state = 1;
+    return true;
+}
+
+// The whole run in launches of the resident sweep, in place in the current copy.
+template <typename T>
+int run_resident(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st) {
+    const RoomHost &h = b->rooms[0];
+    ResidentRun<T> run;
+    run.room = make_room<T>(b, 0);
+    run.layer = h.has_layer;
+    run.walls = h.has_walls;
+    run.n_relax = h.n_relax;
+    run.mailbox = b->resident_mailbox;
+    run.step_base = b->step_base;
+    run.epoch = b->resident_epoch;
+    run.wait_limit_ns = b->test_wait_limit_ns ? b->test_wait_limit_ns : kWaitLimitNs;
+    run.stop_step = b->test_skip_plane;
+    for (int64_t done = 0; done < n_steps;) {
+        int64_t n = std::min(kResidentMaxSteps, n_steps - done);
+        if (n_steps - done - n == 1) n -= 1;      // a launch takes two steps or more
+        run.steps = (int)n;
+        ACF_CUDA(resident_launch<T>(b->resident, run, step_offset + done, st));
+        b->launches += 2;
+        done += n;
+    }
+    ACF_CUDA(cudaGetLastError());
+    return ACF_OK;
+}
+
 template <typename T>
 int run_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st) {
+    if (resident_ready<T>(b, n_steps, st)) return run_resident<T>(b, n_steps, step_offset, st);
     if (b->rooms.size() > 1 && b->room_table_dirty) {
         int rc = upload_room_table<T>(b);
         if (rc) return rc;
@@ -4712,6 +4443,8 @@ void free_batch(acf_batch *b) {
     cudaFree(b->pair_ring);
     cudaFree(b->pair_progress);
     cudaFree(b->psi2);
+    cudaFree(b->resident_mailbox);
+    cudaFree(b->resident_epoch);
     cudaFree(b->state);
     cudaFree(b->room_table);
     cudaFree(b->fused_table);
@@ -5036,8 +4769,8 @@ int pending_status(acf_batch *b) {
         return fail(ACF_ERR_NUMERIC, "a sweep produced a non-finite pressure (NaN or infinity) in "
                     "an earlier run; the state is not valid");
     if (word & kStatusWaitTimeout)
-        return fail(ACF_ERR_STATE, "a staged sweep gave up waiting for its bulk copies in an "
-                    "earlier run; the state is not valid");
+        return fail(ACF_ERR_STATE, "a sweep gave up waiting (a staged sweep for its bulk copies, "
+                    "a resident sweep for its neighbours) in an earlier run; the state is not valid");
     return ACF_OK;
 }
 

@@ -25,7 +25,9 @@ from .medium import AIR
 
 __all__ = ["CudaAcousticFDTD", "DEFAULT_STEPS_PER_GRAPH", "pinned_array"]
 
-#: Steps captured per CUDA graph for long runs; shorter runs launch step by step.
+#: Steps captured per CUDA graph for long runs; shorter runs launch step by step. A room small
+#: enough for the GPU's registers and shared memory takes many steps per launch instead (0 turns
+#: both off).
 DEFAULT_STEPS_PER_GRAPH = 64
 
 
@@ -107,8 +109,8 @@ def raise_for_status(word: int) -> None:
     if word & _native.STATUS_WAIT_TIMEOUT:
         raise _native.NativeError(_native.ERR_STATE, "acf_device_status",
                                   "a sweep timed out waiting (a staged sweep for its bulk "
-                                  "copies, a two-step sweep for its neighbours); the solver "
-                                  "state is not valid")
+                                  "copies, a two-step or resident sweep for its neighbours); the "
+                                  "solver state is not valid")
 
 
 def pinned_array(shape, dtype=np.float32) -> np.ndarray:

@@ -210,17 +210,24 @@ int acf_set_staging(acf_solver *solver, int32_t rows, int32_t stages, int32_t ve
 int acf_device_status(acf_solver *solver, int32_t *status);
 int acf_batch_device_status(acf_batch *batch, int32_t *status);
 
-/* Test hook of the staged and two-step sweeps, for exercising their bounded waits without a
+/* Test hook of the staged, two-step and resident sweeps, for exercising their bounded waits without a
  * fault: every wait gives up after `wait_limit_ns` (0: the built-in two seconds; else 1 ms to
  * two seconds), and with `skip_plane` >= 0 (-1: none) the grid's first CTA withholds something
  * its waiters need. In the staged sweep its producer leaves out the copies of x plane
  * `skip_plane`, so that CTA's consumers wait for data that never arrives, run out of time, raise
  * bit 1 of the status word and return; the producer drains the copies it did issue before the
  * CTA exits. In the two-step sweep it stops publishing its progress from that plane on, so its
- * neighbour CTAs' waits run out, raise bit 1 and stop waiting. No counterpart in the reference. */
+ * neighbour CTAs' waits run out, raise bit 1 and stop waiting; in the resident sweep (see
+ * acf_set_graph) it sends nothing from step `skip_plane` of a run on, with the same effect. No
+ * counterpart in the reference. */
 int acf_set_wait_test(acf_solver *solver, int64_t wait_limit_ns, int32_t skip_plane);
 
-/* Use CUDA graphs of `steps_per_graph` steps for runs at least that long (0 disables). */
+/* Use CUDA graphs of `steps_per_graph` steps for runs at least that long. 0: launch every step by
+ * itself. Otherwise a single room on the two-sweep or fused scheme whose state fits the GPU's
+ * registers and shared memory (up to about 2 million cells in single precision, 900 thousand in
+ * double; fewer with relaxation states) takes runs of 8 steps or more in one cooperative launch
+ * per 2048 steps, with the same results bit for bit; its inboxes (at most 20 MB) are allocated at
+ * the first such run, and where that fails, or inside a stream capture, the sweeps are used. */
 int acf_set_graph(acf_solver *solver, int32_t steps_per_graph);
 
 /* Launch geometry of both sweeps: threads per block (power of two, 32..256) and consecutive
@@ -341,7 +348,8 @@ int acf_profile_enable(acf_solver *solver, int32_t enable);
 int acf_profile_read(acf_solver *solver, double *velocity_ms, double *pressure_ms,
                      int64_t *launches);
 
-/* Kernels launched by this handle since creation (sweeps, graph replays counted per kernel). */
+/* Kernels launched by this handle since creation (sweeps, graph replays counted per kernel; a
+ * launch that takes many steps counts once). */
 int64_t acf_launch_count(const acf_solver *solver);
 
 /* ---- Impulse-response post-processing (FP64, on the device) ----------------------------
