@@ -45,8 +45,10 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <deque>
 #include <mutex>
 #include <new>
+#include <unordered_map>
 #include <vector>
 
 #include "acfdtd_b200.h"
@@ -3411,6 +3413,165 @@ struct DeviceGuard {
     }
 };
 
+// Device memory of the handles. A program that makes a solver per room (an impulse response per
+// position, a sweep over designs) otherwise pays cudaMalloc and cudaFree (350 to 700 us each here,
+// 20 of them per solver) and a pinned word (3 ms) more than for the run: blocks given back are kept
+// for the next handle of this process, at most kCacheBytes of them in all (the oldest go first), and
+// every one is freed before an allocation is reported as failed. A block is given back only
+// once the device is idle, as cudaFree itself waits, so the next owner may use it on any stream.
+constexpr size_t kCacheBytes = (size_t)256 << 20;
+
+struct BlockCache {
+    struct Block {
+        void *pointer;
+        size_t bytes;
+        int device;
+    };
+    std::mutex lock;
+    std::unordered_map<void *, Block> used;
+    std::deque<Block> idle;        // oldest first
+    size_t idle_bytes = 0;
+
+    // Free idle blocks, oldest first, until at most `keep` bytes remain.
+    void trim(size_t keep) {
+        while (idle_bytes > keep && !idle.empty()) {
+            const Block b = idle.front();
+            idle.pop_front();
+            idle_bytes -= b.bytes;
+            DeviceGuard guard(b.device);
+            cudaFree(b.pointer);
+        }
+    }
+};
+
+BlockCache &block_cache() {
+    static BlockCache *cache = new BlockCache;   // outlives every handle, also at process exit
+    return *cache;
+}
+
+cudaError_t dev_malloc_bytes(void **out, size_t bytes) {
+    BlockCache &cache = block_cache();
+    int device = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err != cudaSuccess) return err;
+    bytes = (std::max<size_t>(bytes, 1) + 511) / 512 * 512;
+    std::lock_guard<std::mutex> hold(cache.lock);
+    // the smallest idle block of this device that fits and wastes at most an eighth
+    size_t best = cache.idle.size();
+    for (size_t n = 0; n < cache.idle.size(); n++) {
+        const BlockCache::Block &b = cache.idle[n];
+        if (b.device == device && b.bytes >= bytes && b.bytes <= bytes + bytes / 8 &&
+            (best == cache.idle.size() || b.bytes < cache.idle[best].bytes))
+            best = n;
+    }
+    BlockCache::Block block{nullptr, bytes, device};
+    if (best < cache.idle.size()) {
+        block = cache.idle[best];
+        cache.idle.erase(cache.idle.begin() + (std::ptrdiff_t)best);
+        cache.idle_bytes -= block.bytes;
+    } else {
+        err = cudaMalloc(&block.pointer, bytes);
+        if (err == cudaErrorMemoryAllocation && cache.idle_bytes > 0) {
+            cudaGetLastError();
+            cache.trim(0);
+            err = cudaMalloc(&block.pointer, bytes);
+        }
+        if (err != cudaSuccess) return err;
+    }
+    cache.used[block.pointer] = block;
+    *out = block.pointer;
+    return cudaSuccess;
+}
+
+template <typename T>
+cudaError_t dev_malloc(T **out, size_t bytes) {
+    void *p = nullptr;
+    const cudaError_t err = dev_malloc_bytes(&p, bytes);
+    if (err == cudaSuccess) *out = (T *)p;
+    return err;
+}
+
+void dev_free(void *pointer) {
+    if (!pointer) return;
+    BlockCache &cache = block_cache();
+    BlockCache::Block block;
+    {
+        std::lock_guard<std::mutex> hold(cache.lock);
+        const auto at = cache.used.find(pointer);
+        if (at == cache.used.end()) return;
+        block = at->second;
+        cache.used.erase(at);
+    }
+    DeviceGuard guard(block.device);
+    if (block.bytes > kCacheBytes / 4 || cudaDeviceSynchronize() != cudaSuccess) {
+        cudaFree(pointer);
+        return;
+    }
+    std::lock_guard<std::mutex> hold(cache.lock);
+    cache.idle.push_back(block);
+    cache.idle_bytes += block.bytes;
+    cache.trim(kCacheBytes);
+}
+
+// The handles' status words in pinned host memory: pages of words, a page freed with its last
+// word except the first, which stays.
+struct PinnedWords {
+    static constexpr int kPerPage = 1024;
+    struct Page {
+        int32_t *words = nullptr;
+        int used = 0;
+        bool taken[kPerPage] = {};
+    };
+    std::mutex lock;
+    std::vector<Page *> pages;
+};
+
+PinnedWords &pinned_words() {
+    static PinnedWords *words = new PinnedWords;
+    return *words;
+}
+
+cudaError_t pinned_word(int32_t **out) {
+    PinnedWords &all = pinned_words();
+    std::lock_guard<std::mutex> hold(all.lock);
+    PinnedWords::Page *page = nullptr;
+    for (PinnedWords::Page *p : all.pages)
+        if (p->used < PinnedWords::kPerPage) page = p;
+    if (!page) {
+        page = new PinnedWords::Page;
+        const cudaError_t err = cudaHostAlloc((void **)&page->words, PinnedWords::kPerPage * sizeof(int32_t),
+                                              cudaHostAllocPortable);
+        if (err != cudaSuccess) {
+            delete page;
+            return err;
+        }
+        all.pages.push_back(page);
+    }
+    int n = 0;
+    while (page->taken[n]) n++;
+    page->taken[n] = true;
+    page->used++;
+    *out = page->words + n;
+    return cudaSuccess;
+}
+
+void release_pinned_word(int32_t *word) {
+    if (!word) return;
+    PinnedWords &all = pinned_words();
+    std::lock_guard<std::mutex> hold(all.lock);
+    for (size_t n = 0; n < all.pages.size(); n++) {
+        PinnedWords::Page *p = all.pages[n];
+        if (word < p->words || word >= p->words + PinnedWords::kPerPage) continue;
+        p->taken[word - p->words] = false;
+        if (--p->used == 0 && n > 0) {
+            cudaFreeHost(p->words);
+            all.pages.erase(all.pages.begin() + (std::ptrdiff_t)n);
+            delete p;
+        }
+        return;
+    }
+}
+
 inline int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
 // Everything the host keeps about one room of a batch.
@@ -3679,7 +3840,7 @@ template <typename T>
 int upload_room_table(acf_batch *b) {
     std::vector<Room<T>> table(b->rooms.size());
     for (size_t r = 0; r < b->rooms.size(); r++) table[r] = make_room<T>(b, (int)r);
-    if (!b->room_table) ACF_CUDA(cudaMalloc(&b->room_table, table.size() * sizeof(Room<T>)));
+    if (!b->room_table) ACF_CUDA(dev_malloc(&b->room_table, table.size() * sizeof(Room<T>)));
     ACF_CUDA(cudaMemcpy(b->room_table, table.data(), table.size() * sizeof(Room<T>), cudaMemcpyHostToDevice));
     if (b->scheme == ACF_SCHEME_FUSED) {
         // Both parities: entry [parity * rooms + r] reads the copy that is current at that parity.
@@ -3699,7 +3860,7 @@ int upload_room_table(acf_batch *b) {
                 f.nvz = (T *)b->other_ptr((int)r, ACF_FIELD_VZ);
                 h.cur = saved;
             }
-        if (!b->fused_table) ACF_CUDA(cudaMalloc(&b->fused_table, fused.size() * sizeof(FusedParams<T>)));
+        if (!b->fused_table) ACF_CUDA(dev_malloc(&b->fused_table, fused.size() * sizeof(FusedParams<T>)));
         ACF_CUDA(cudaMemcpy(b->fused_table, fused.data(), fused.size() * sizeof(FusedParams<T>),
                             cudaMemcpyHostToDevice));
     }
@@ -3727,9 +3888,9 @@ int build_tiles(acf_batch *b) {
             }
     }
     if (tiles.size() > (size_t)INT32_MAX) return fail(ACF_ERR_ARGUMENT, "too many tiles");
-    cudaFree(b->tiles);
+    dev_free(b->tiles);
     b->tiles = nullptr;
-    ACF_CUDA(cudaMalloc(&b->tiles, std::max<size_t>(1, tiles.size()) * sizeof(Tile)));
+    ACF_CUDA(dev_malloc(&b->tiles, std::max<size_t>(1, tiles.size()) * sizeof(Tile)));
     ACF_CUDA(cudaMemcpy(b->tiles, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice));
     b->n_tiles = (int32_t)tiles.size();
     // ctas_per_sm == 0: one CTA per tile, scheduled by the hardware; otherwise a persistent
@@ -3971,14 +4132,14 @@ int set_time_blocking(acf_batch *b, int32_t steps) {
     const size_t ring_bytes = (size_t)groups * kPairRing * h.plane * sizeof(float);
     const size_t counters = (size_t)(per_group * groups);
     b->time_block = 1;          // until the new buffers are in place
-    cudaFree(b->pair_ring);
-    cudaFree(b->pair_progress);
+    dev_free(b->pair_ring);
+    dev_free(b->pair_progress);
     b->pair_ring = nullptr;
     b->pair_progress = nullptr;
-    ACF_CUDA(cudaMalloc(&b->pair_ring, ring_bytes));
-    ACF_CUDA(cudaMalloc(&b->pair_progress, counters * sizeof(int32_t)));
+    ACF_CUDA(dev_malloc(&b->pair_ring, ring_bytes));
+    ACF_CUDA(dev_malloc(&b->pair_progress, counters * sizeof(int32_t)));
     if (h.n_relax > 0 && !b->psi2)
-        ACF_CUDA(cudaMalloc(&b->psi2, (size_t)h.n_relax * h.field * sizeof(float)));
+        ACF_CUDA(dev_malloc(&b->psi2, (size_t)h.n_relax * h.field * sizeof(float)));
     b->pair_grid = dim3(gx, gy, (unsigned)groups);
     b->pair_block = dim3(bx, by, 1);
     b->pair_planes = planes;
@@ -4176,8 +4337,8 @@ bool resident_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
     const RoomHost &h = b->rooms[0];
     b->resident = resident_plan<T>(h.nx, h.ny, h.nz, h.n_relax, h.has_layer, b->sms, (size_t)b->smem_per_block);
     if (b->resident.planes == 0) return false;
-    if (cudaMalloc(&b->resident_mailbox, b->resident.mailbox_bytes) != cudaSuccess ||
-        cudaMalloc(&b->resident_epoch, 2 * sizeof(uint32_t)) != cudaSuccess ||
+    if (dev_malloc(&b->resident_mailbox, b->resident.mailbox_bytes) != cudaSuccess ||
+        dev_malloc(&b->resident_epoch, 2 * sizeof(uint32_t)) != cudaSuccess ||
         cudaMemsetAsync(b->resident_mailbox, 0, b->resident.mailbox_bytes, st) != cudaSuccess ||
         cudaMemsetAsync(b->resident_epoch, 0, 2 * sizeof(uint32_t), st) != cudaSuccess) {
         cudaGetLastError();
@@ -4388,27 +4549,28 @@ int upload_cast(void **dst, const std::vector<double> &host, size_t es) {
     std::vector<char> cast(std::max<size_t>(1, host.size()) * es, 0);
     if (es == 4) cast_copy<float>(cast.data(), host.data(), host.size());
     else cast_copy<double>(cast.data(), host.data(), host.size());
-    ACF_CUDA(cudaMalloc(dst, cast.size()));
+    ACF_CUDA(dev_malloc(dst, cast.size()));
     ACF_CUDA(cudaMemcpy(*dst, cast.data(), cast.size(), cudaMemcpyHostToDevice));
     return ACF_OK;
 }
 
 void free_room(RoomHost &h) {
-    cudaFree(h.second);
-    cudaFree(h.profiles);
-    cudaFree(h.shell);
-    cudaFree(h.src_off);
-    cudaFree(h.src_len);
-    cudaFree(h.src_sig);
-    cudaFree(h.rec_off);
-    cudaFree(h.rec_start);
-    cudaFree(h.rec);
+    dev_free(h.second);
+    dev_free(h.profiles);
+    dev_free(h.shell);
+    dev_free(h.src_off);
+    dev_free(h.src_len);
+    dev_free(h.src_sig);
+    dev_free(h.rec_off);
+    dev_free(h.rec_start);
+    dev_free(h.rec);
     h = RoomHost();
 }
 
 void free_batch(acf_batch *b) {
     if (!b) return;
     DeviceGuard guard(b->device);
+    cudaDeviceSynchronize();       // nothing of this handle is in flight when its memory goes
     if (b->graph) cudaGraphExecDestroy(b->graph);
     if (b->graph_odd) cudaGraphExecDestroy(b->graph_odd);
     b->g_record.release();
@@ -4419,38 +4581,38 @@ void free_batch(acf_batch *b) {
     for (auto &e : b->ring)
         if (e) cudaEventDestroy(e);
     if (b->status_event) cudaEventDestroy(b->status_event);
-    if (b->status_host) cudaFreeHost(b->status_host);
+    release_pinned_word(b->status_host);
     for (auto &r : b->rooms) free_room(r);
-    cudaFree(b->adj.hist_shell);
-    cudaFree(b->adj.checkpoints);
-    cudaFree(b->adj.scratch);
-    cudaFree(b->adj.segment);
-    cudaFree(b->adj.fields);
-    cudaFree(b->adj.fields2);
-    cudaFree(b->adj.grad_shell);
-    cudaFree(b->adj.air_partials);
-    cudaFree(b->adj.grad_rec);
-    cudaFree(b->adj.grad_src);
+    dev_free(b->adj.hist_shell);
+    dev_free(b->adj.checkpoints);
+    dev_free(b->adj.scratch);
+    dev_free(b->adj.segment);
+    dev_free(b->adj.fields);
+    dev_free(b->adj.fields2);
+    dev_free(b->adj.grad_shell);
+    dev_free(b->adj.air_partials);
+    dev_free(b->adj.grad_rec);
+    dev_free(b->adj.grad_src);
     for (auto &ra : b->badj) {
-        cudaFree(ra.hist_shell);
-        cudaFree(ra.fields);
-        cudaFree(ra.fields2);
-        cudaFree(ra.grad_shell);
-        cudaFree(ra.grad_rec);
-        cudaFree(ra.grad_src);
+        dev_free(ra.hist_shell);
+        dev_free(ra.fields);
+        dev_free(ra.fields2);
+        dev_free(ra.grad_shell);
+        dev_free(ra.grad_rec);
+        dev_free(ra.grad_src);
     }
-    cudaFree(b->badj_table);
-    cudaFree(b->pair_ring);
-    cudaFree(b->pair_progress);
-    cudaFree(b->psi2);
-    cudaFree(b->resident_mailbox);
-    cudaFree(b->resident_epoch);
-    cudaFree(b->state);
-    cudaFree(b->room_table);
-    cudaFree(b->fused_table);
-    cudaFree(b->tiles);
-    cudaFree(b->step_base);
-    cudaFree(b->energy_scratch);
+    dev_free(b->badj_table);
+    dev_free(b->pair_ring);
+    dev_free(b->pair_progress);
+    dev_free(b->psi2);
+    dev_free(b->resident_mailbox);
+    dev_free(b->resident_epoch);
+    dev_free(b->state);
+    dev_free(b->room_table);
+    dev_free(b->fused_table);
+    dev_free(b->tiles);
+    dev_free(b->step_base);
+    dev_free(b->energy_scratch);
     delete b;
 }
 
@@ -4532,7 +4694,7 @@ int create_batch(int32_t n_rooms, const acf_config *configs, acf_batch *b) {
     if (const char *inject = getenv("ACF_INJECT_ALLOC_FAILURE"); inject && *inject && strcmp(inject, "0") != 0)
         return fail(ACF_ERR_MEMORY, "cudaMalloc of %zu bytes of state failed (injected by "
                     "ACF_INJECT_ALLOC_FAILURE)", b->state_bytes);
-    if (cudaMalloc(&b->state, b->state_bytes) != cudaSuccess)
+    if (dev_malloc(&b->state, b->state_bytes) != cudaSuccess)
         return fail(ACF_ERR_MEMORY, "cudaMalloc of %zu bytes of state failed", b->state_bytes);
     ACF_CUDA(cudaMemset(b->state, 0, b->state_bytes));
 
@@ -4579,10 +4741,10 @@ int create_batch(int32_t n_rooms, const acf_config *configs, acf_batch *b) {
         }
     }
 
-    if (cudaMalloc(&b->step_base, 2 * sizeof(int64_t)) != cudaSuccess)
+    if (dev_malloc(&b->step_base, 2 * sizeof(int64_t)) != cudaSuccess)
         return fail(ACF_ERR_MEMORY, "cudaMalloc of step counter failed");
     ACF_CUDA(cudaMemset(b->step_base, 0, 2 * sizeof(int64_t)));
-    if (cudaHostAlloc((void **)&b->status_host, sizeof(int32_t), cudaHostAllocDefault) != cudaSuccess)
+    if (pinned_word(&b->status_host) != cudaSuccess)
         return fail(ACF_ERR_MEMORY, "pinned status word allocation failed");
     *b->status_host = 0;
     ACF_CUDA(cudaEventCreateWithFlags(&b->status_event, cudaEventDisableTiming));
@@ -4590,9 +4752,8 @@ int create_batch(int32_t n_rooms, const acf_config *configs, acf_batch *b) {
     cudaDeviceGetAttribute(&b->smem_per_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
     b->energy_blocks = 4 * b->sms;
     const size_t scratch = ((size_t)b->energy_blocks + 1) * kEnergyTerms * sizeof(double);
-    if (cudaMalloc(&b->energy_scratch, scratch) != cudaSuccess)
+    if (dev_malloc(&b->energy_scratch, scratch) != cudaSuccess)
         return fail(ACF_ERR_MEMORY, "cudaMalloc of energy scratch failed");
-    for (auto &ev : b->ring) ACF_CUDA(cudaEventCreate(&ev));
     if (batched) {
         // one CTA per tile of 128 (row, chunk) pairs x 8 planes: the best measured schedule on
         // uneven-room batches (persistent grids lose to the hardware scheduler here)
@@ -4632,9 +4793,9 @@ int set_sources(acf_batch *b, int room, int64_t n, const int64_t *cell, const in
         len[q] = length[q];
     }
     ACF_CUDA(cudaDeviceSynchronize());
-    cudaFree(h.src_off);
-    cudaFree(h.src_len);
-    cudaFree(h.src_sig);
+    dev_free(h.src_off);
+    dev_free(h.src_len);
+    dev_free(h.src_sig);
     h.src_off = h.src_len = nullptr;
     h.src_sig = nullptr;
     h.n_src = 0;
@@ -4644,8 +4805,8 @@ int set_sources(acf_batch *b, int room, int64_t n, const int64_t *cell, const in
     const size_t es = b->elem();
     // padded offsets, then their in-plane offsets
     for (int64_t q = 0; q < n; q++) off.push_back(off[q] % h.plane);
-    ACF_CUDA(cudaMalloc(&h.src_off, 2 * n * sizeof(int64_t)));
-    ACF_CUDA(cudaMalloc(&h.src_len, n * sizeof(int64_t)));
+    ACF_CUDA(dev_malloc(&h.src_off, 2 * n * sizeof(int64_t)));
+    ACF_CUDA(dev_malloc(&h.src_len, n * sizeof(int64_t)));
     ACF_CUDA(cudaMemcpy(h.src_off, off.data(), 2 * n * sizeof(int64_t), cudaMemcpyHostToDevice));
     ACF_CUDA(cudaMemcpy(h.src_len, len.data(), n * sizeof(int64_t), cudaMemcpyHostToDevice));
     std::vector<double> host((size_t)n * (size_t)std::max<int64_t>(stride, 1), 0.0);
@@ -4685,16 +4846,16 @@ int set_receivers(acf_batch *b, int room, int64_t n, const int64_t *cell, const 
     const size_t es = b->elem();
     if (n > 0 && h.rec_capacity > 0 && n != h.n_rec) {
         void *grown = nullptr;
-        ACF_CUDA(cudaMalloc(&grown, (size_t)n * h.rec_capacity * es));
+        ACF_CUDA(dev_malloc(&grown, (size_t)n * h.rec_capacity * es));
         ACF_CUDA(cudaMemset(grown, 0, (size_t)n * h.rec_capacity * es));
         const int64_t keep = std::min<int64_t>(n, h.n_rec);
         if (keep > 0 && h.rec)
             ACF_CUDA(cudaMemcpy(grown, h.rec, (size_t)keep * h.rec_capacity * es, cudaMemcpyDeviceToDevice));
-        cudaFree(h.rec);
+        dev_free(h.rec);
         h.rec = grown;
     }
-    cudaFree(h.rec_off);
-    cudaFree(h.rec_start);
+    dev_free(h.rec_off);
+    dev_free(h.rec_start);
     h.rec_off = h.rec_start = nullptr;
     h.n_rec = 0;
     b->graph_dirty = b->adj_graphs_dirty = true;
@@ -4702,8 +4863,8 @@ int set_receivers(acf_batch *b, int room, int64_t n, const int64_t *cell, const 
     h.host_rec_start.assign(start_step, start_step + n);
     if (n == 0) return ACF_OK;
     for (int64_t r = 0; r < n; r++) off.push_back(off[r] % h.plane);   // then in-plane offsets
-    ACF_CUDA(cudaMalloc(&h.rec_off, 2 * n * sizeof(int64_t)));
-    ACF_CUDA(cudaMalloc(&h.rec_start, n * sizeof(int64_t)));
+    ACF_CUDA(dev_malloc(&h.rec_off, 2 * n * sizeof(int64_t)));
+    ACF_CUDA(dev_malloc(&h.rec_start, n * sizeof(int64_t)));
     ACF_CUDA(cudaMemcpy(h.rec_off, off.data(), 2 * n * sizeof(int64_t), cudaMemcpyHostToDevice));
     ACF_CUDA(cudaMemcpy(h.rec_start, start_step, n * sizeof(int64_t), cudaMemcpyHostToDevice));
     h.n_rec = n;
@@ -4741,12 +4902,12 @@ int ensure_recording(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStr
         const size_t es = b->elem();
         void *grown = nullptr;
         ACF_CUDA(cudaStreamSynchronize(st));
-        ACF_CUDA(cudaMalloc(&grown, (size_t)h.n_rec * cap * es));
+        ACF_CUDA(dev_malloc(&grown, (size_t)h.n_rec * cap * es));
         ACF_CUDA(cudaMemset(grown, 0, (size_t)h.n_rec * cap * es));
         if (h.rec && h.rec_capacity > 0)
             ACF_CUDA(cudaMemcpy2D(grown, (size_t)cap * es, h.rec, (size_t)h.rec_capacity * es,
                                   (size_t)h.rec_capacity * es, (size_t)h.n_rec, cudaMemcpyDeviceToDevice));
-        cudaFree(h.rec);
+        dev_free(h.rec);
         h.rec = grown;
         h.rec_capacity = cap;
         b->graph_dirty = b->adj_graphs_dirty = true;
@@ -5161,6 +5322,11 @@ int device_status(acf_batch *b, int32_t *status) {
 
 int profile_enable(acf_batch *b, int32_t enable) {
     if (!b) return fail(ACF_ERR_ARGUMENT, "null handle");
+    if (enable) {
+        DeviceGuard guard(b->device);
+        for (auto &ev : b->ring)
+            if (!ev) ACF_CUDA(cudaEventCreate(&ev));
+    }
     b->profiling = enable != 0;
     b->prof_velocity_ms = b->prof_pressure_ms = 0;
     b->prof_launches = 0;
@@ -5240,7 +5406,7 @@ int set_scheme(acf_batch *b, int32_t scheme) {
         for (RoomHost &h : b->rooms) {
             if (h.second) continue;
             const size_t bytes = ((size_t)4 * h.field + (size_t)h.pz) * b->elem();
-            if (cudaMalloc(&h.second, bytes) != cudaSuccess)
+            if (dev_malloc(&h.second, bytes) != cudaSuccess)
                 return fail(ACF_ERR_MEMORY, "cudaMalloc of %zu bytes for the fused scheme failed", bytes);
             ACF_CUDA(cudaMemset(h.second, 0, bytes));
         }
@@ -5493,7 +5659,7 @@ int forward_record_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cuda
     if (lean && !b->rooms[0].second) {
         RoomHost &h = b->rooms[0];
         const size_t bytes = ((size_t)4 * h.field + (size_t)h.pz) * b->elem();
-        if (cudaMalloc(&h.second, bytes) != cudaSuccess) {
+        if (dev_malloc(&h.second, bytes) != cudaSuccess) {
             cudaGetLastError();
             h.second = nullptr;
             lean = false;
@@ -5535,17 +5701,17 @@ int adjoint_impl(acf_batch *b, const double *grad_rec, double *grad_src, double 
     // graphs stay valid from call to call.
     const int64_t cap = A.capacity;
     if (h.n_rec > A.grad_rows_rec || !A.grad_rec) {
-        cudaFree(A.grad_rec);
+        dev_free(A.grad_rec);
         A.grad_rec = nullptr;
         A.grad_rows_rec = std::max<int64_t>(1, h.n_rec);
-        ACF_CUDA(cudaMalloc(&A.grad_rec, (size_t)A.grad_rows_rec * cap * sizeof(double)));
+        ACF_CUDA(dev_malloc(&A.grad_rec, (size_t)A.grad_rows_rec * cap * sizeof(double)));
         b->adj_graphs_dirty = true;
     }
     if (h.n_src > A.grad_rows_src || !A.grad_src) {
-        cudaFree(A.grad_src);
+        dev_free(A.grad_src);
         A.grad_src = nullptr;
         A.grad_rows_src = std::max<int64_t>(1, h.n_src);
-        ACF_CUDA(cudaMalloc(&A.grad_src, (size_t)A.grad_rows_src * cap * sizeof(double)));
+        ACF_CUDA(dev_malloc(&A.grad_src, (size_t)A.grad_rows_src * cap * sizeof(double)));
         b->adj_graphs_dirty = true;
     }
     if (h.n_rec > 0)
@@ -5562,9 +5728,9 @@ int adjoint_impl(acf_batch *b, const double *grad_rec, double *grad_src, double 
     const int NA = 3 * h.n_relax + 1;
     if (air) {
         if (A.air_blocks < blocks) {
-            cudaFree(A.air_partials);
+            dev_free(A.air_partials);
             A.air_partials = nullptr;
-            ACF_CUDA(cudaMalloc(&A.air_partials, (size_t)blocks * NA * sizeof(double)));
+            ACF_CUDA(dev_malloc(&A.air_partials, (size_t)blocks * NA * sizeof(double)));
             A.air_blocks = blocks;
             b->adj_graphs_dirty = true;
         }
@@ -5753,6 +5919,10 @@ int adjoint_prepare(acf_batch *b, int32_t flags, int64_t max_steps, int32_t ever
         const RoomHost &h = b->rooms[0];
         const double whole = (double)max_steps * (1 + h.n_relax) * h.field * b->elem();
         size_t free_bytes = 0, total_bytes = 0;
+        {
+            std::lock_guard<std::mutex> hold(block_cache().lock);
+            block_cache().trim(0);
+        }
         ACF_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
         every = whole <= 0.6 * (double)free_bytes ? (int32_t)std::min<int64_t>(max_steps, INT32_MAX)
                                                    : (int32_t)std::ceil(std::sqrt((double)max_steps));
@@ -5761,10 +5931,10 @@ int adjoint_prepare(acf_batch *b, int32_t flags, int64_t max_steps, int32_t ever
     b->adj_graphs_dirty = true;
     void **buffers[] = {&A.hist_shell, &A.checkpoints, &A.scratch, &A.segment, &A.fields, &A.fields2};
     for (void **p : buffers) {
-        cudaFree(*p);
+        dev_free(*p);
         *p = nullptr;
     }
-    cudaFree(A.grad_shell);
+    dev_free(A.grad_shell);
     A.grad_shell = nullptr;
     const RoomHost &h = b->rooms[0];
     const size_t es = b->elem();
@@ -5782,25 +5952,25 @@ int adjoint_prepare(acf_batch *b, int32_t flags, int64_t max_steps, int32_t ever
         A.shell_total += sizes[q];
     }
     const size_t adj_bytes = ((size_t)(5 + h.n_relax) * h.field + h.pz) * es;
-    ACF_CUDA(cudaMalloc(&A.fields, adj_bytes));
+    ACF_CUDA(dev_malloc(&A.fields, adj_bytes));
     const size_t second = ((size_t)4 * h.field + h.pz) * es;
-    ACF_CUDA(cudaMalloc(&A.fields2, second));
+    ACF_CUDA(dev_malloc(&A.fields2, second));
     ACF_CUDA(cudaMemset(A.fields2, 0, second));
     if ((flags & ACF_GRAD_WALLS) && h.has_walls) {
         const size_t bytes = (size_t)max_steps * A.shell_total * 2 * es;
-        if (cudaMalloc(&A.hist_shell, bytes) != cudaSuccess)
+        if (dev_malloc(&A.hist_shell, bytes) != cudaSuccess)
             return fail(ACF_ERR_MEMORY, "cudaMalloc of %zu bytes of wall history failed", bytes);
-        ACF_CUDA(cudaMalloc(&A.grad_shell, A.shell_total * sizeof(double)));
+        ACF_CUDA(dev_malloc(&A.grad_shell, A.shell_total * sizeof(double)));
     }
     if ((flags & ACF_GRAD_AIR) && h.n_relax > 0) {
         const int64_t n_ckpt = (max_steps + every - 1) / every;
         const size_t block = b->room_block_bytes(0);
-        if (cudaMalloc(&A.checkpoints, (size_t)n_ckpt * block) != cudaSuccess)
+        if (dev_malloc(&A.checkpoints, (size_t)n_ckpt * block) != cudaSuccess)
             return fail(ACF_ERR_MEMORY, "cudaMalloc of %lld checkpoints failed", (long long)n_ckpt);
-        ACF_CUDA(cudaMalloc(&A.scratch, block + (size_t)h.pz * es));
+        ACF_CUDA(dev_malloc(&A.scratch, block + (size_t)h.pz * es));
         ACF_CUDA(cudaMemset(A.scratch, 0, block + (size_t)h.pz * es));
         const size_t seg = ((size_t)every * (1 + h.n_relax) * h.field + h.pz) * es;
-        if (cudaMalloc(&A.segment, seg) != cudaSuccess)
+        if (dev_malloc(&A.segment, seg) != cudaSuccess)
             return fail(ACF_ERR_MEMORY, "cudaMalloc of %zu bytes of segment history failed", seg);
         ACF_CUDA(cudaMemset(A.segment, 0, seg));
     }
@@ -5895,12 +6065,12 @@ int batch_adjoint_prepare(acf_batch *b, int64_t max_steps) {
     DeviceGuard guard(b->device);
     ACF_CUDA(cudaDeviceSynchronize());
     for (auto &ra : b->badj) {
-        cudaFree(ra.hist_shell);
-        cudaFree(ra.fields);
-        cudaFree(ra.fields2);
-        cudaFree(ra.grad_shell);
-        cudaFree(ra.grad_rec);
-        cudaFree(ra.grad_src);
+        dev_free(ra.hist_shell);
+        dev_free(ra.fields);
+        dev_free(ra.fields2);
+        dev_free(ra.grad_shell);
+        dev_free(ra.grad_rec);
+        dev_free(ra.grad_src);
     }
     b->badj.assign(b->rooms.size(), acf_batch::RoomAdjoint());
     const size_t es = b->elem();
@@ -5914,12 +6084,12 @@ int batch_adjoint_prepare(acf_batch *b, int64_t max_steps) {
             ra.shell_total += sizes[q];
         }
         const size_t hist = (size_t)max_steps * ra.shell_total * 2 * es;
-        if (cudaMalloc(&ra.hist_shell, hist) != cudaSuccess)
+        if (dev_malloc(&ra.hist_shell, hist) != cudaSuccess)
             return fail(ACF_ERR_MEMORY, "room %zu: cudaMalloc of %zu bytes of wall history failed", r, hist);
-        ACF_CUDA(cudaMalloc(&ra.fields, ((size_t)(5 + h.n_relax) * h.field + h.pz) * es));
-        ACF_CUDA(cudaMalloc(&ra.fields2, ((size_t)4 * h.field + h.pz) * es));
+        ACF_CUDA(dev_malloc(&ra.fields, ((size_t)(5 + h.n_relax) * h.field + h.pz) * es));
+        ACF_CUDA(dev_malloc(&ra.fields2, ((size_t)4 * h.field + h.pz) * es));
         ACF_CUDA(cudaMemset(ra.fields2, 0, ((size_t)4 * h.field + h.pz) * es));
-        ACF_CUDA(cudaMalloc(&ra.grad_shell, ra.shell_total * sizeof(double)));
+        ACF_CUDA(dev_malloc(&ra.grad_shell, ra.shell_total * sizeof(double)));
     }
     b->badj_capacity = max_steps;
     b->badj_recorded = 0;
@@ -5975,7 +6145,7 @@ int upload_adjoint_table(acf_batch *b, int64_t n) {
         o.out_d = a.ld;
         (void)n;
     }
-    if (!b->badj_table) ACF_CUDA(cudaMalloc(&b->badj_table, table.size() * sizeof(AdjointParams<T>)));
+    if (!b->badj_table) ACF_CUDA(dev_malloc(&b->badj_table, table.size() * sizeof(AdjointParams<T>)));
     ACF_CUDA(cudaMemcpy(b->badj_table, table.data(), table.size() * sizeof(AdjointParams<T>),
                         cudaMemcpyHostToDevice));
     return ACF_OK;
@@ -6025,14 +6195,14 @@ int batch_adjoint_impl(acf_batch *b, const double *grad_rec, double *grad_src, d
         const RoomHost &h = b->rooms[r];
         auto &ra = b->badj[r];
         if (h.n_rec > ra.rows_rec || !ra.grad_rec) {
-            cudaFree(ra.grad_rec);
+            dev_free(ra.grad_rec);
             ra.rows_rec = std::max<int64_t>(1, h.n_rec);
-            ACF_CUDA(cudaMalloc(&ra.grad_rec, (size_t)ra.rows_rec * cap * sizeof(double)));
+            ACF_CUDA(dev_malloc(&ra.grad_rec, (size_t)ra.rows_rec * cap * sizeof(double)));
         }
         if (h.n_src > ra.rows_src || !ra.grad_src) {
-            cudaFree(ra.grad_src);
+            dev_free(ra.grad_src);
             ra.rows_src = std::max<int64_t>(1, h.n_src);
-            ACF_CUDA(cudaMalloc(&ra.grad_src, (size_t)ra.rows_src * cap * sizeof(double)));
+            ACF_CUDA(dev_malloc(&ra.grad_src, (size_t)ra.rows_src * cap * sizeof(double)));
         }
         if (h.n_rec > 0)
             ACF_CUDA(cudaMemcpy2DAsync(ra.grad_rec, cap * sizeof(double), grad_rec + rec_row * n,
@@ -6598,12 +6768,12 @@ int acf_forward_record(acf_solver *h, int64_t n_steps, int64_t step_offset, acf_
         const size_t es = h->elem();
         void *grown = nullptr;
         ACF_CUDA(cudaStreamSynchronize(st));
-        ACF_CUDA(cudaMalloc(&grown, (size_t)r.n_rec * cap * es));
+        ACF_CUDA(dev_malloc(&grown, (size_t)r.n_rec * cap * es));
         ACF_CUDA(cudaMemset(grown, 0, (size_t)r.n_rec * cap * es));
         if (r.rec && r.rec_capacity > 0)
             ACF_CUDA(cudaMemcpy2D(grown, (size_t)cap * es, r.rec, (size_t)r.rec_capacity * es,
                                   (size_t)r.rec_capacity * es, (size_t)r.n_rec, cudaMemcpyDeviceToDevice));
-        cudaFree(r.rec);
+        dev_free(r.rec);
         r.rec = grown;
         r.rec_capacity = cap;
         h->graph_dirty = h->adj_graphs_dirty = true;
@@ -6758,12 +6928,12 @@ int acf_batch_forward_record(acf_batch *b, int64_t n_steps, int64_t step_offset,
         const size_t es = b->elem();
         void *grown = nullptr;
         ACF_CUDA(cudaStreamSynchronize(st));
-        ACF_CUDA(cudaMalloc(&grown, (size_t)r.n_rec * cap * es));
+        ACF_CUDA(dev_malloc(&grown, (size_t)r.n_rec * cap * es));
         ACF_CUDA(cudaMemset(grown, 0, (size_t)r.n_rec * cap * es));
         if (r.rec && r.rec_capacity > 0)
             ACF_CUDA(cudaMemcpy2D(grown, (size_t)cap * es, r.rec, (size_t)r.rec_capacity * es,
                                   (size_t)r.rec_capacity * es, (size_t)r.n_rec, cudaMemcpyDeviceToDevice));
-        cudaFree(r.rec);
+        dev_free(r.rec);
         r.rec = grown;
         r.rec_capacity = cap;
         b->graph_dirty = b->adj_graphs_dirty = true;
