@@ -53,18 +53,18 @@
 
 #include "acfdtd_b200.h"
 #include "acfdtd_device.cuh"
+#include "acfdtd_host.cuh"
 #include "acfdtd_resident.cuh"
 
 using namespace acf;
 
 namespace {
 
-constexpr int kRowAlign = 8;       // row pitch granularity, elements
-constexpr int kEnergyTerms = 7;
-
 thread_local char g_last_error[512] = "";
 
-int fail(int code, const char *fmt, ...) {
+}  // namespace
+
+int acf::fail(int code, const char *fmt, ...) {
     va_list args;
     va_start(args, fmt);
     vsnprintf(g_last_error, sizeof(g_last_error), fmt, args);
@@ -72,13 +72,10 @@ int fail(int code, const char *fmt, ...) {
     return code;
 }
 
-#define ACF_CUDA(call)                                                                     \
-    do {                                                                                   \
-        cudaError_t err__ = (call);                                                        \
-        if (err__ != cudaSuccess)                                                          \
-            return fail(ACF_ERR_CUDA, "%s failed: %s (%s:%d)", #call,                      \
-                        cudaGetErrorString(err__), __FILE__, __LINE__);                    \
-    } while (0)
+namespace {
+
+constexpr int kRowAlign = 8;       // row pitch granularity, elements
+constexpr int kEnergyTerms = 7;
 
 template <typename T>
 struct StepParams {
@@ -6261,220 +6258,6 @@ int batch_adjoint_impl(acf_batch *b, const double *grad_rec, double *grad_src, d
     return ACF_OK;
 }
 
-// ------------------------------------------------------------------------------------------
-// Impulse-response post-processing in FP64 (ac-fdtd src/ac_fdtd/metrics.py:57-111 and the
-// spectral division of src/ac_fdtd/sources.py:80-108): the steps after the time loop, on the
-// receiver signals where the recordings already are. One CTA per channel; every sum in FP64.
-
-constexpr int kPostThreads = 1024;
-
-// Exclusive scan of one double per thread over the CTA (kPostThreads threads, thread order);
-// `shared` holds 32 doubles. Returns the sum of the values of the threads before this one;
-// *total gets the CTA's sum.
-__device__ double block_exclusive_scan(double v, double *shared, double *total) {
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double inclusive = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const double up = __shfl_up_sync(0xffffffffu, inclusive, d);
-        if (lane >= (unsigned)d) inclusive += up;
-    }
-    double within = __shfl_up_sync(0xffffffffu, inclusive, 1);
-    if (lane == 0) within = 0.0;
-    if (lane == 31) shared[warp] = inclusive;
-    __syncthreads();
-    if (warp == 0) {
-        double w = shared[lane];
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const double up = __shfl_up_sync(0xffffffffu, w, d);
-            if (lane >= (unsigned)d) w += up;
-        }
-        shared[lane] = w;
-    }
-    __syncthreads();
-    const double before = warp > 0 ? shared[warp - 1] : 0.0;
-    *total = shared[31];
-    __syncthreads();
-    return lane == 0 ? before : before + within;
-}
-
-__device__ double block_sum(double v, double *shared) {
-    double total;
-    block_exclusive_scan(v, shared, &total);
-    return total;
-}
-
-__device__ int64_t block_min(int64_t v, int64_t *shared) {
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) v = min(v, (int64_t)__shfl_xor_sync(0xffffffffu, v, d));
-    if (lane == 0) shared[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        int64_t w = shared[lane];
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) w = min(w, (int64_t)__shfl_xor_sync(0xffffffffu, w, d));
-        if (lane == 0) shared[0] = w;
-    }
-    __syncthreads();
-    const int64_t out = shared[0];
-    __syncthreads();
-    return out;
-}
-
-// Schroeder's backward integral I(k) = sum_{m >= k} h(m)^2, as 10 log10 max(I(k) / I(0),
-// 1e-300) floored at `floor_db` (metrics.py:57-69). Thread t owns a contiguous run of the
-// reversed signal; one CTA scan of the runs' sums gives each run's starting value.
-__global__ void __launch_bounds__(kPostThreads) schroeder_decay_kernel(const double *response, int64_t n,
-                                                                       double floor_db, double *decay) {
-    __shared__ double shared[32];
-    const double *h = response + (int64_t)blockIdx.x * n;
-    double *out = decay + (int64_t)blockIdx.x * n;
-    const int64_t run = (n + kPostThreads - 1) / kPostThreads;
-    const int64_t q0 = min((int64_t)threadIdx.x * run, n), q1 = min(q0 + run, n);
-    double mine = 0.0;
-    for (int64_t q = q0; q < q1; q++) {
-        const double x = h[n - 1 - q];
-        mine += x * x;
-    }
-    double sum_all;
-    const double start = block_exclusive_scan(mine, shared, &sum_all);   // the later runs in time
-    // The curve is normalised by I(0) itself, as the reference divides by its first entry: the
-    // thread holding sample 0 forms it with the same additions as its pass below, so the first
-    // level is exactly 0 dB.
-    __shared__ double first;
-    if (q0 < n && q1 == n) {
-        double running = start;
-        for (int64_t q = q0; q < q1; q++) {
-            const double x = h[n - 1 - q];
-            running += x * x;
-        }
-        first = running;
-    }
-    __syncthreads();
-    const double total = first;
-    double running = start;
-    for (int64_t q = q0; q < q1; q++) {
-        const double x = h[n - 1 - q];
-        running += x * x;
-        const double level = 10.0 * log10(fmax(running / total, 1e-300));
-        out[n - 1 - q] = fmax(level, floor_db);
-    }
-}
-
-// Seconds per 60 dB from a least-squares line through the decay curve between the first sample
-// at or below `upper` dB and the first at or below `lower` dB (metrics.py:72-84); NaN and
-// `failed[c] = 1` when the curve does not reach `lower` after `upper`, where the reference
-// raises.
-__global__ void __launch_bounds__(kPostThreads) decay_fit_kernel(const double *decay, int64_t n,
-                                                                 double sample_rate, double upper,
-                                                                 double lower, double *seconds,
-                                                                 int32_t *failed) {
-    __shared__ double shared[32];
-    __shared__ int64_t ishared[32];
-    const double *d = decay + (int64_t)blockIdx.x * n;
-    int64_t first_upper = n, first_lower = n;
-    for (int64_t k = threadIdx.x; k < n; k += kPostThreads) {
-        const double v = d[k];
-        if (v <= upper && k < first_upper) first_upper = k;
-        if (v <= lower && k < first_lower) first_lower = k;
-    }
-    int64_t start = block_min(first_upper, ishared), end = block_min(first_lower, ishared);
-    if (start == n) start = 0;   // numpy.argmax of an all-false mask
-    if (end == n) end = 0;
-    if (end <= start) {
-        if (threadIdx.x == 0) {
-            seconds[blockIdx.x] = __longlong_as_double(0x7ff8000000000000ll);
-            failed[blockIdx.x] = 1;
-        }
-        return;
-    }
-    const double m = (double)(end - start);
-    double sx = 0.0, sy = 0.0;
-    for (int64_t k = start + threadIdx.x; k < end; k += kPostThreads) {
-        sx += (double)k / sample_rate;
-        sy += d[k];
-    }
-    const double mean_x = block_sum(sx, shared) / m, mean_y = block_sum(sy, shared) / m;
-    double sxy = 0.0, sxx = 0.0;
-    for (int64_t k = start + threadIdx.x; k < end; k += kPostThreads) {
-        const double x = (double)k / sample_rate - mean_x;
-        sxy += x * (d[k] - mean_y);
-        sxx += x * x;
-    }
-    const double slope = block_sum(sxy, shared) / block_sum(sxx, shared);
-    if (threadIdx.x == 0) {
-        seconds[blockIdx.x] = -60.0 / slope;
-        failed[blockIdx.x] = 0;
-    }
-}
-
-// Early-to-late energy ratio in dB with the split at sample `boundary` (metrics.py:104-110).
-__global__ void __launch_bounds__(kPostThreads) clarity_kernel(const double *response, int64_t n,
-                                                               int64_t boundary, double *db) {
-    __shared__ double shared[32];
-    const double *h = response + (int64_t)blockIdx.x * n;
-    double early = 0.0, late = 0.0;
-    for (int64_t k = threadIdx.x; k < n; k += kPostThreads) {
-        const double e = h[k] * h[k];
-        if (k < boundary) early += e;
-        else late += e;
-    }
-    early = block_sum(early, shared);
-    late = block_sum(late, shared);
-    if (threadIdx.x == 0) db[blockIdx.x] = 10.0 * log10(early / late);
-}
-
-// Largest |S(f)|^2 of the excitation's spectrum (the regularisation's scale).
-__global__ void __launch_bounds__(kPostThreads) spectrum_peak_power(const double2 *source, int64_t bins,
-                                                                   double *peak) {
-    __shared__ double shared[32];
-    double best = 0.0;
-    for (int64_t k = threadIdx.x; k < bins; k += kPostThreads) {
-        const double a = hypot(source[k].x, source[k].y);
-        best = fmax(best, a * a);
-    }
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, d));
-    if (lane == 0) shared[warp] = best;
-    __syncthreads();
-    if (warp == 0) {
-        double w = shared[lane];
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) w = fmax(w, __shfl_xor_sync(0xffffffffu, w, d));
-        if (lane == 0) *peak = w;
-    }
-}
-
-// R(f) = X(f) conj(S(f)) / (|S(f)|^2 + reg * max |S|^2), zero above max_frequency, for every
-// channel's spectrum X (sources.py:103-107). Bin k is at k * bin_hz, as numpy.fft.rfftfreq.
-__global__ void spectral_divide_kernel(const double2 *spectra, const double2 *source, int64_t channels,
-                                       int64_t bins, double bin_hz, double max_frequency,
-                                       double regularisation, const double *peak, double2 *out) {
-    const int64_t at = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (at >= channels * bins) return;
-    const int64_t k = at % bins;
-    double2 r = make_double2(0.0, 0.0);
-    if (!((double)k * bin_hz > max_frequency)) {
-        const double2 x = spectra[at], src = source[k];
-        const double a = hypot(src.x, src.y);
-        const double denominator = a * a + regularisation * *peak;
-        // x * conj(src): (x.x src.x - x.y (-src.y)) + (x.x (-src.y) + x.y src.x) i
-        const double re = x.x * src.x - x.y * -src.y;
-        const double im = x.x * -src.y + x.y * src.x;
-        r = make_double2(re / denominator, im / denominator);
-    }
-    out[at] = r;
-}
-
-int check_post_args(const void *a, const void *b, int64_t channels, int64_t n) {
-    if (!a || !b) return fail(ACF_ERR_ARGUMENT, "null device array");
-    if (channels < 1 || channels > 65535 || n < 1) return fail(ACF_ERR_ARGUMENT, "need 1..65535 channels of at least one sample");
-    return ACF_OK;
-}
-
 }  // namespace
 
 // ==========================================================================================
@@ -7004,52 +6787,6 @@ int acf_energy_terms_noalloc(const void *p, const void *vx, const void *vy, cons
                                                            (const float *)vy, (const float *)vz,
                                                            nx, ny, nz, inv_dx, scratch);
     energy_finish<<<1, 32, 0, st>>>(scratch, nx + 1, terms_device);
-    ACF_CUDA(cudaGetLastError());
-    return ACF_OK;
-}
-
-int acf_schroeder_decay(const double *response, int64_t channels, int64_t n, double floor_db,
-                        double *decay, acf_stream stream) {
-    int rc = check_post_args(response, decay, channels, n);
-    if (rc) return rc;
-    schroeder_decay_kernel<<<(unsigned)channels, kPostThreads, 0, (cudaStream_t)stream>>>(response, n, floor_db, decay);
-    ACF_CUDA(cudaGetLastError());
-    return ACF_OK;
-}
-
-int acf_decay_fit(const double *decay, int64_t channels, int64_t n, double sample_rate, double upper_db,
-                  double lower_db, double *seconds, int32_t *failed, acf_stream stream) {
-    int rc = check_post_args(decay, seconds, channels, n);
-    if (rc) return rc;
-    if (!failed) return fail(ACF_ERR_ARGUMENT, "null device array");
-    if (!(sample_rate > 0.0)) return fail(ACF_ERR_ARGUMENT, "sample rate must be positive");
-    decay_fit_kernel<<<(unsigned)channels, kPostThreads, 0, (cudaStream_t)stream>>>(decay, n, sample_rate, upper_db,
-                                                                                lower_db, seconds, failed);
-    ACF_CUDA(cudaGetLastError());
-    return ACF_OK;
-}
-
-int acf_clarity(const double *response, int64_t channels, int64_t n, int64_t boundary, double *db,
-                acf_stream stream) {
-    int rc = check_post_args(response, db, channels, n);
-    if (rc) return rc;
-    clarity_kernel<<<(unsigned)channels, kPostThreads, 0, (cudaStream_t)stream>>>(response, n, boundary, db);
-    ACF_CUDA(cudaGetLastError());
-    return ACF_OK;
-}
-
-int acf_spectral_divide(const void *spectra, const void *source, int64_t channels, int64_t bins,
-                        double bin_hz, double max_frequency, double regularisation, double *scratch,
-                        void *out, acf_stream stream) {
-    int rc = check_post_args(spectra, source, channels, bins);
-    if (rc) return rc;
-    if (!scratch || !out) return fail(ACF_ERR_ARGUMENT, "null device array");
-    cudaStream_t st = (cudaStream_t)stream;
-    spectrum_peak_power<<<1, kPostThreads, 0, st>>>((const double2 *)source, bins, scratch);
-    const int64_t total = channels * bins;
-    spectral_divide_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
-        (const double2 *)spectra, (const double2 *)source, channels, bins, bin_hz, max_frequency,
-        regularisation, scratch, (double2 *)out);
     ACF_CUDA(cudaGetLastError());
     return ACF_OK;
 }
