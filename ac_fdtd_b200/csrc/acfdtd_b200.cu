@@ -54,6 +54,7 @@
 #include "acfdtd_b200.h"
 #include "acfdtd_device.cuh"
 #include "acfdtd_host.cuh"
+#include "acfdtd_fused64.cuh"
 #include "acfdtd_resident.cuh"
 
 using namespace acf;
@@ -344,15 +345,6 @@ __device__ __forceinline__ void pressure_column(const Room<T> &s, int i_begin, i
 // then its pressure. Per cell and step this moves (8 + 2R) elements instead of (12 + 2R); every
 // value is produced by the same operations as in the two sweeps, so the results are identical.
 
-template <typename T>
-struct FusedParams {
-    Room<T> room;                  // p, vx, vy, vz: current state (read); psi updated in place
-    T *np, *nvx, *nvy, *nvz;       // next state (written), same geometry
-    const int64_t *step_base;
-    int32_t local_step;
-    int32_t planes;
-};
-
 template <typename T, bool LAYER>
 __device__ __forceinline__ T damp3(T v, T fa, T fb, T fc) {
     if (LAYER) {
@@ -529,24 +521,6 @@ __device__ __forceinline__ void fused_column(const FusedParams<T> &f, int i_begi
         }
     }
     report_nonfinite(s.status, bad != bad);
-}
-
-// Resident blocks of 256 threads the compiler must fit (register budget 65536 / (256 x this)).
-// For the fp32 room with a layer: 80 registers, no spills. Timed at 384^3 with the plane
-// prefetch, 72 registers (56 bytes of spills) ran 2 % slower and 64 (140 bytes) 19 % slower.
-#ifndef ACF_FUSED_MIN_BLOCKS
-#define ACF_FUSED_MIN_BLOCKS(T, LAYER, NR) (sizeof(T) == 8 ? 2 : (LAYER || NR >= 4 ? 3 : 4))
-#endif
-
-template <typename T, bool LAYER, bool WALLS, int NR>
-__global__ void __launch_bounds__(256, ACF_FUSED_MIN_BLOCKS(T, LAYER, NR)) fused_sweep(const FusedParams<T> f) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (c >= f.room.nchunks || j >= f.room.ny) return;
-    const bool any_point = (f.room.n_src | f.room.n_rec) != 0;
-    const int64_t step = any_point ? (*f.step_base + f.local_step) : 0;
-    const int i_begin = blockIdx.z * f.planes;
-    fused_column<T, LAYER, WALLS, NR>(f, i_begin, min(f.room.nx, i_begin + f.planes), j, c, step);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -3948,13 +3922,6 @@ struct BatchPressure {
 };
 
 template <typename T, bool L, bool W, int NR>
-struct FusedStep {
-    static void launch(const FusedParams<T> &p, dim3 g, dim3 b, cudaStream_t st) {
-        fused_sweep<T, L, W, NR><<<g, b, 0, st>>>(p);
-    }
-};
-
-template <typename T, bool L, bool W, int NR>
 struct LeanStep {
     static void launch(const LeanParams &p, dim3 g, dim3 b, cudaStream_t st) {
         lean_sweep<L, W, NR><<<g, b, 0, st>>>(p);
@@ -4270,7 +4237,7 @@ void launch_step(acf_batch *b, int32_t local, cudaStream_t st, cudaEvent_t *even
                     dispatch_pressure<float, LeanStepPadded>(h.has_layer, h.has_walls, h.n_relax, g, L.grid,
                                                              L.block, st);
             } else {
-                dispatch_pressure<T, FusedStep>(h.has_layer, h.has_walls, h.n_relax, f, L.grid, L.block, st);
+                launch_pack_sweep(f, h.has_layer, h.has_walls, h.n_relax, b->block_threads, st);
             }
         }
         h.cur ^= 1;
@@ -5051,7 +5018,7 @@ void fused_slab_step(acf_batch *const *parts, int n, const int32_t *own_lo, cons
                 dispatch_pressure<float, LeanStepPadded>(h.has_layer, h.has_walls, h.n_relax, lp, L.grid,
                                                          L.block, streams[q]);
         } else {
-            dispatch_pressure<T, FusedStep>(h.has_layer, h.has_walls, h.n_relax, f[q], L.grid, L.block, streams[q]);
+            launch_pack_sweep(f[q], h.has_layer, h.has_walls, h.n_relax, parts[q]->block_threads, streams[q]);
         }
         parts[q]->launches += 1;
         after(q);

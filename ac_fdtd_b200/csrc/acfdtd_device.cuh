@@ -167,6 +167,17 @@ struct History {
     int32_t reserved;
 };
 
+// A fused step: the velocity and pressure updates of a step in one sweep, from the current copy of
+// p and v into the next.
+template <typename T>
+struct FusedParams {
+    Room<T> room;                  // p, vx, vy, vz: current state (read); psi updated in place
+    T *np, *nvx, *nvy, *nvz;       // next state (written), same geometry
+    const int64_t *step_base;
+    int32_t local_step;
+    int32_t planes;
+};
+
 // ------------------------------------------------------------------------------------------
 // Walls, sources and receivers of one (row, chunk) column.
 
