@@ -3617,6 +3617,8 @@ struct acf_batch {
     // graphs (index: parity of the fused scheme's current buffer at the start of a replay)
     int32_t graph_steps = 0;
     cudaGraphExec_t graph = nullptr, graph_odd = nullptr;
+    cudaGraphExec_t graph_one = nullptr;   // the two-sweep scheme's steps as fused steps (one_sweep)
+    int one_sweep_state = 0;               // 0 undecided, 1 the second copy is there, -1 not
     cudaStream_t capture_stream = nullptr;
     bool graph_dirty = true;
 
@@ -4338,6 +4340,46 @@ int run_resident(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_
     return ACF_OK;
 }
 
+// Whether a run of the two-sweep scheme takes its steps in pairs of fused steps, which end in the
+// room's own copy: (8 + 2R) elements moved per cell instead of (12 + 2R). In double precision the
+// fused step is the faster one at every size that is not held on chip (112^3 19.3 against 27.3 us,
+// 203 x 187 x 211 with every term 155 against 208). In single precision the sweeps are as fast or
+// faster while the state fits L2 (walls only: 160 x 161 x 163 34 against 38 us, 67 MB of state;
+// 176^3 47 against 42 us, 87 MB; 251 x 240 x 263 with every term 201 against 166), so from 0.6 of L2
+// on. It takes a second copy of p and v, so only where that is at most a sixteenth of the
+// device memory free at the first such run, and in place otherwise.
+constexpr double kOneSweepL2 = 0.6;
+constexpr int64_t kOneSweepMinSteps = 8;
+
+bool one_sweep_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
+    if (b->one_sweep_state < 0 || n_steps < kOneSweepMinSteps || b->scheme != ACF_SCHEME_TWO_SWEEPS ||
+        b->rooms.size() != 1 || b->profiling || b->graph_steps == 0)
+        return false;
+    RoomHost &h = b->rooms[0];
+    if (b->precision == 4 && (double)b->room_block_bytes(0) < kOneSweepL2 * (double)b->l2_bytes) return false;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    if (b->one_sweep_state == 0) {
+        b->one_sweep_state = -1;
+        if (!h.second) {
+            const size_t bytes = ((size_t)4 * h.field + (size_t)h.pz) * b->elem();
+            size_t free_bytes = 0, total_bytes = 0;
+            if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess || bytes > free_bytes / 16 ||
+                dev_malloc(&h.second, bytes) != cudaSuccess) {
+                cudaGetLastError();
+                h.second = nullptr;
+                return false;
+            }
+            if (cudaMemsetAsync(h.second, 0, bytes, st) != cudaSuccess) return false;
+        }
+        b->one_sweep_state = 1;
+    }
+    return true;
+}
+
 template <typename T>
 int run_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st) {
     if (resident_ready<T>(b, n_steps, st)) return run_resident<T>(b, n_steps, step_offset, st);
@@ -4400,6 +4442,20 @@ int run_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st
         }
     }
 
+    // The two-sweep scheme's steps as fused steps: an even number of them, then the sweeps for an odd
+    // step, so that the state is in the room's own copy before and after.
+    const bool one_sweep = one_sweep_ready(b, n_steps, st);
+    const bool last_in_place = one_sweep && n_steps % 2 != 0;
+    struct Scheme {                        // the scheme while the launches below are queued
+        acf_batch *b;
+        int own;
+        ~Scheme() { b->scheme = own; }
+    } scheme{b, b->scheme};
+    if (one_sweep) {
+        b->scheme = ACF_SCHEME_FUSED;
+        n_steps -= last_in_place ? 1 : 0;
+    }
+
     int64_t done = 0;
     if (b->pressure_only() && b->po_first) {
         // The step from the p-v state is not the repeated one: launch it before any graph.
@@ -4415,12 +4471,13 @@ int run_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st
     const int kernels_per_step = fused ? 1 : 2;
     if (G > 0 && n_steps >= G) {
         if (b->graph_dirty) {
-            if (b->graph) cudaGraphExecDestroy(b->graph);
-            if (b->graph_odd) cudaGraphExecDestroy(b->graph_odd);
-            b->graph = b->graph_odd = nullptr;
+            for (cudaGraphExec_t *g : {&b->graph, &b->graph_odd, &b->graph_one}) {
+                if (*g) cudaGraphExecDestroy(*g);
+                *g = nullptr;
+            }
             b->graph_dirty = false;
         }
-        cudaGraphExec_t &exec = (fused && b->rooms[0].cur) ? b->graph_odd : b->graph;
+        cudaGraphExec_t &exec = one_sweep ? b->graph_one : (fused && b->rooms[0].cur) ? b->graph_odd : b->graph;
         if (!exec) {
             if (!b->capture_stream)
                 ACF_CUDA(cudaStreamCreateWithFlags(&b->capture_stream, cudaStreamNonBlocking));
@@ -4442,6 +4499,11 @@ int run_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st
     for (int64_t t = 0; done + t < n_steps; t++) {
         launch_step<T>(b, (int32_t)t, st, nullptr);
         b->launches += kernels_per_step;
+    }
+    if (last_in_place) {
+        b->scheme = scheme.own;
+        launch_step<T>(b, (int32_t)(n_steps - done), st, nullptr);
+        b->launches += 2;
     }
     ACF_CUDA(cudaGetLastError());
     return ACF_OK;
@@ -4537,6 +4599,7 @@ void free_batch(acf_batch *b) {
     cudaDeviceSynchronize();       // nothing of this handle is in flight when its memory goes
     if (b->graph) cudaGraphExecDestroy(b->graph);
     if (b->graph_odd) cudaGraphExecDestroy(b->graph_odd);
+    if (b->graph_one) cudaGraphExecDestroy(b->graph_one);
     b->g_record.release();
     b->g_recompute.release();
     b->g_adjoint.release();

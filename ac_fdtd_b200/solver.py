@@ -573,7 +573,8 @@ class CudaAcousticFDTD:
         sweep into a second copy of p and v) or ``"staged"`` (the fused sweep with its inputs
         streamed into shared memory by bulk copies). Results are bit-identical; the fused steps
         move (8 + 2R) elements per cell instead of (12 + 2R) and need four more fields of
-        memory. ``"pressure_only"``: the second-order wave equation on p alone (rigid or
+        memory (a long run on ``"two_sweeps"`` takes fused steps inside where that is faster and the
+        second copy is a small part of the free memory). ``"pressure_only"``: the second-order wave equation on p alone (rigid or
         impedance walls, no absorbing layer or air absorption), 3 elements per cell and step;
         its first step is the p-v step from the state as it stands, so pressures and recordings
         equal the other schemes' to rounding, and from then on no velocities are kept
