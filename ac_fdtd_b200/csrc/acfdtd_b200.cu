@@ -54,7 +54,7 @@
 #include "acfdtd_b200.h"
 #include "acfdtd_device.cuh"
 #include "acfdtd_host.cuh"
-#include "acfdtd_fused64.cuh"
+#include "acfdtd_fused.cuh"
 #include "acfdtd_resident.cuh"
 
 using namespace acf;
@@ -85,12 +85,6 @@ struct StepParams {
     const int64_t *step_base;      // absolute step of local step 0, in device memory
     int32_t local_step;
     int32_t planes;                // consecutive x planes marched by one block
-};
-
-// One unit of work of a batched sweep: up to blockDim.x consecutive (row, chunk) pairs of one
-// room, over the x planes [i_begin, i_end).
-struct Tile {
-    int32_t room, first, count, i_begin, i_end, reserved;
 };
 
 template <typename T>
@@ -355,174 +349,6 @@ __device__ __forceinline__ T damp3(T v, T fa, T fb, T fc) {
     return v;
 }
 
-template <typename T, bool LAYER, bool WALLS, int NR>
-__device__ __forceinline__ void fused_column(const FusedParams<T> &f, int i_begin, int i_end, int j,
-                                             int c, int64_t step) {
-    const Room<T> &s = f.room;
-    const int k0 = c * kVec;
-    const T cv = s.cv, cp = s.cp;
-    const bool any_point = (s.n_src | s.n_rec) != 0;
-    const int64_t column = (int64_t)j * s.pz + k0;
-    const bool has_above = k0 + kVec < s.nz;   // p and vz at k0 + 4 are interior
-    bool all_points = false;
-    const uint32_t points = any_point ? column_points(s, j, k0, all_points) : 0u;
-    const bool any_mine = points != 0 || all_points;
-    const bool wall_column = j == 0 || j == s.ny - 1 || k0 == 0 || k0 + kVec >= s.nz;
-
-    // Layer profiles are read where used (L1-resident): holding the z profiles of the chunk
-    // across the march would cost registers the load phase needs.
-    T fj_cell = T(1), fj_face = T(1), fj1_face = T(1);
-    if (LAYER) {
-        fj_cell = __ldg(s.cell[1] + j);
-        fj_face = __ldg(s.face[1] + j);
-        fj1_face = __ldg(s.face[1] + j + 1);
-    }
-
-    // Carried from plane to plane: p(i) and the updated vx on face i.
-    T P[kVec], XL[kVec];
-    T bad = T(0);   // NaN once a pressure this column produced is not finite
-    {
-        const int64_t base = (int64_t)i_begin * s.plane + column;
-        Vec4<T>::ldg(s.p + base, P);
-        T V[kVec], Q[kVec];
-        Vec4<T>::ldg(s.vx + base, V);
-        if (i_begin > 0) Vec4<T>::ldg(s.p + base - s.plane, Q);
-        const T fi_face = LAYER ? __ldg(s.face[0] + i_begin) : T(1);
-#pragma unroll
-        for (int e = 0; e < kVec; e++) {
-            T v = V[e];
-            if (i_begin > 0) v = v - cv * (P[e] - Q[e]);
-            XL[e] = damp3<T, LAYER>(v, fi_face, fj_cell,
-                                    LAYER ? __ldg(s.cell[2] + min(k0 + e, s.nz - 1)) : T(1));
-        }
-    }
-
-    for (int i = i_begin; i < i_end; i++) {
-        const int64_t base = (int64_t)i * s.plane + column;
-        const bool x_inner = i + 1 < s.nx;
-        // ---- the next plane's own-row inputs into L2 (its y-neighbour rows are other
-        // threads' own rows): the loads of the next iteration then wait on L2, not DRAM.
-        if (s.prefetch && i + 1 < i_end) {
-            const int64_t next = base + s.plane;
-            if (i + 2 < s.nx) prefetch_l2(s.p + next + s.plane);
-            prefetch_l2(s.vx + next + s.plane);
-            prefetch_l2(s.vy + next);
-            prefetch_l2(s.vz + next);
-#pragma unroll
-            for (int r = 0; r < NR; r++) prefetch_l2(s.psi + r * s.field + next);
-        }
-        // ---- loads (all read-only: the next state goes to the other buffer)
-        T PX[kVec], VXo[kVec], PYm[kVec], PYp[kVec], VY[kVec], VYp[kVec], VZ[kVec], S[NR > 0 ? NR : 1][kVec];
-        if (x_inner) Vec4<T>::ldg(s.p + base + s.plane, PX);
-        Vec4<T>::ldg(s.vx + base + s.plane, VXo);
-        if (j > 0) Vec4<T>::ldg(s.p + base - s.pz, PYm);
-        if (j + 1 < s.ny) Vec4<T>::ldg(s.p + base + s.pz, PYp);
-        Vec4<T>::ldg(s.vy + base, VY);
-        Vec4<T>::ldg(s.vy + base + s.pz, VYp);
-        Vec4<T>::ldg(s.vz + base, VZ);
-        const T p_below = k0 > 0 ? __ldg(s.p + base - 1) : T(0);
-        const T p_above = has_above ? __ldg(s.p + base + kVec) : T(0);
-        const T vz_above = k0 + kVec <= s.nz ? __ldg(s.vz + base + kVec) : T(0);
-#pragma unroll
-        for (int r = 0; r < NR; r++) Vec4<T>::load(s.psi + r * s.field + base, S[r]);
-        T fi_cell = T(1), fi1_face = T(1);
-        if (LAYER) {
-            fi_cell = __ldg(s.cell[0] + i);
-            fi1_face = __ldg(s.face[0] + i + 1);
-        }
-
-        // ---- updated faces: x upper (carried on), y lower and upper, z lower and upper
-        T XH[kVec], YL[kVec], YH[kVec], ZL[kVec];
-#pragma unroll
-        for (int e = 0; e < kVec; e++) {
-            const T fkc = LAYER ? __ldg(s.cell[2] + min(k0 + e, s.nz - 1)) : T(1);
-            T v = VXo[e];
-            if (x_inner) v = v - cv * (PX[e] - P[e]);
-            XH[e] = damp3<T, LAYER>(v, fi1_face, fj_cell, fkc);
-            v = VY[e];
-            if (j > 0) v = v - cv * (P[e] - PYm[e]);
-            YL[e] = damp3<T, LAYER>(v, fi_cell, fj_face, fkc);
-            v = VYp[e];
-            if (j + 1 < s.ny) v = v - cv * (PYp[e] - P[e]);
-            YH[e] = damp3<T, LAYER>(v, fi_cell, fj1_face, fkc);
-            const int k = k0 + e;
-            v = VZ[e];
-            if (k > 0 && k < s.nz) v = v - cv * (P[e] - (e == 0 ? p_below : P[e - 1]));
-            ZL[e] = damp3<T, LAYER>(v, fi_cell, fj_cell,
-                                    LAYER ? __ldg(s.face[2] + min(k0 + e, s.nz)) : T(1));
-        }
-        // z face k0 + 4: the next chunk's first lower face, or the top face z = nz.
-        T ZH3 = vz_above;
-        if (has_above) ZH3 = ZH3 - cv * (p_above - P[kVec - 1]);
-        ZH3 = damp3<T, LAYER>(ZH3, fi_cell, fj_cell,
-                              LAYER ? __ldg(s.face[2] + min(k0 + kVec, s.nz)) : T(1));
-
-        // ---- pressure, as the pressure sweep computes it
-        const bool boundary = wall_column || i == 0 || i == s.nx - 1;
-        T Pn[kVec];
-#pragma unroll
-        for (int e = 0; e < kVec; e++) {
-            const int k = k0 + e;
-            T pe = P[e];
-            if (k < s.nz) {
-                const T zh = e + 1 < kVec ? ZL[e + 1] : ZH3;
-                T d = XH[e] - XL[e];
-                d = d + (YH[e] - YL[e]);
-                d = d + (zh - ZL[e]);
-#pragma unroll
-                for (int r = 0; r < NR; r++) {
-                    const T target = d * s.gain[r];
-                    const T offset = S[r][e] - target;
-                    S[r][e] = offset * s.decay[r] + target;
-                    pe = pe + offset * s.mean[r];
-                }
-                if (NR > 0) pe = pe + d * s.relax_scale;
-                pe = pe - d * cp;
-                if (WALLS && boundary) {
-                    T fu, fp;
-                    if (wall_pair(s, i, j, k, fu, fp)) pe = pe * fu - P[e] * fp;
-                }
-                if (LAYER) {
-                    pe = pe * fi_cell;
-                    pe = pe * fj_cell;
-                    pe = pe * __ldg(s.cell[2] + k);
-                }
-            }
-            Pn[e] = pe;
-        }
-        if (any_mine) add_sources(s, points, all_points, base, k0, step, Pn);
-#pragma unroll
-        for (int e = 0; e < kVec; e++) bad = finite_acc(bad, Pn[e]);
-
-        // ---- stores: p, the three lower faces, the far boundary faces, psi in place. A z
-        // element k == nz inside this chunk is the top face, already updated in ZL (no
-        // gradient, damped by face profile nz); elements past it are padding.
-        T ZS[kVec];
-#pragma unroll
-        for (int e = 0; e < kVec; e++) ZS[e] = k0 + e <= s.nz ? ZL[e] : VZ[e];
-        // A slab's ghost planes get their p from the neighbours' sweeps, never from their own;
-        // its boundary planes also go to the neighbours' ghost planes (in their next copies).
-        if (i >= s.own_lo && i < s.own_hi) Vec4<T>::store(f.np + base, Pn);
-        if (s.ghost_lo != nullptr && i == s.own_lo) Vec4<T>::store(s.ghost_lo + column, Pn);
-        if (s.ghost_hi != nullptr && i == s.own_hi - 1) Vec4<T>::store(s.ghost_hi + column, Pn);
-        Vec4<T>::store(f.nvx + base, XL);
-        Vec4<T>::store(f.nvy + base, YL);
-        Vec4<T>::store(f.nvz + base, ZS);
-        if (i == s.nx - 1) Vec4<T>::store(f.nvx + base + s.plane, XH);
-        if (j == s.ny - 1) Vec4<T>::store(f.nvy + base + s.pz, YH);
-        if (k0 + kVec == s.nz) f.nvz[base + kVec] = ZH3;
-#pragma unroll
-        for (int r = 0; r < NR; r++) Vec4<T>::store(s.psi + r * s.field + base, S[r]);
-        if (any_mine) record_receivers(s, points, all_points, base, step, Pn);
-#pragma unroll
-        for (int e = 0; e < kVec; e++) {
-            XL[e] = XH[e];
-            P[e] = PX[e];
-        }
-    }
-    report_nonfinite(s.status, bad != bad);
-}
-
 // ------------------------------------------------------------------------------------------
 // The fused step with its inputs staged in shared memory by the bulk-copy engine.
 //
@@ -536,7 +362,7 @@ __device__ __forceinline__ void fused_column(const FusedParams<T> &f, int i_begi
 // registers the arithmetic needs. A thread owns VW = 2 or 4 consecutive z elements of one row:
 // shared memory per thread is what bounds the warps an SM holds (the ring takes about 70 bytes
 // per thread and stage at VW = 2), so the narrower vector keeps twice as many warps resident
-// to hide the arithmetic's latency. The arithmetic is fused_column's, element for element, so
+// to hide the arithmetic's latency. The arithmetic is the fused step's, element for element, so
 // the results are identical to the two-sweep and fused schemes.
 //
 // The copies are issued by a producer warp of their own. Consumer warps release a buffer through
@@ -809,7 +635,7 @@ fused_staged_sweep(const StagedParams<T> g) {
         __syncthreads();
     }
     const int np = any_point ? n_points : 0;
-    const bool overflow = np > kStagedPointCap;   // too many: scan every point, as fused_column
+    const bool overflow = np > kStagedPointCap;   // too many: scan every point, as column_points
 
     const int c = tid % g.block_x;
     const int ry = tid / g.block_x;
@@ -840,7 +666,7 @@ fused_staged_sweep(const StagedParams<T> g) {
 #pragma unroll
             for (int e = 0; e <= VW; e++) fkf[e] = __ldg(s.face[2] + min(k0 + e, s.nz));
         }
-        // The updated vx on face i_begin, as fused_column starts its march.
+        // The updated vx on face i_begin, where the march starts.
         const int64_t base = (int64_t)i_begin * s.plane + column;
         T P0[VW], V[VW], Q[VW];
         VecW<T, VW>::ldg(s.p + base, P0);
@@ -2218,45 +2044,6 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 8 ? 2 : 3)) pressure_batch(
     }
 }
 
-// (a)+(b) over a batch: the fused step (fused_column) on the same tile table, each CTA staging
-// the fused parameters of its tile's room -- the room description with the current p and v and
-// the next copy to write -- for the parity all rooms are at.
-template <typename T>
-struct FusedBatchParams {
-    const FusedParams<T> *rooms;   // one per room, for the current parity
-    const Tile *tiles;
-    int32_t n_tiles;
-    int32_t local_step;
-    const int64_t *step_base;
-};
-
-// 96 registers (fp32): measured best on 64 uneven rooms against 80 (spills) and 128 (fewer warps).
-template <typename T, bool LAYER, bool WALLS, int NR>
-__global__ void __maxnreg__(sizeof(T) == 8 ? 168 : 96) fused_batch(const FusedBatchParams<T> b) {
-    __shared__ __align__(16) unsigned char raw[sizeof(FusedParams<T>)];
-    FusedParams<T> *room = reinterpret_cast<FusedParams<T> *>(raw);
-    static_assert(sizeof(FusedParams<T>) % sizeof(int) == 0, "FusedParams must be a whole number of words");
-    const int64_t step = *b.step_base + b.local_step;
-    int staged = -1;
-    for (int t = blockIdx.x; t < b.n_tiles; t += gridDim.x) {
-        const Tile tile = b.tiles[t];
-        if (tile.room != staged) {
-            __syncthreads();
-            const int *from = reinterpret_cast<const int *>(b.rooms + tile.room);
-            int *to = reinterpret_cast<int *>(raw);
-            for (int w = threadIdx.x; w < (int)(sizeof(FusedParams<T>) / sizeof(int)); w += blockDim.x)
-                to[w] = __ldg(from + w);
-            __syncthreads();
-            staged = tile.room;
-        }
-        if ((int)threadIdx.x < tile.count) {
-            const int pair = tile.first + threadIdx.x;
-            fused_column<T, LAYER, WALLS, NR>(*room, tile.i_begin, tile.i_end, pair / room->room.nchunks,
-                                              pair % room->room.nchunks, step);
-        }
-    }
-}
-
 // ------------------------------------------------------------------------------------------
 // Adjoint: the transposed leapfrog, run backward in time (single rooms).
 //
@@ -3596,6 +3383,8 @@ struct acf_batch {
     bool room_table_dirty = true;
     Tile *tiles = nullptr;
     int32_t n_tiles = 0;
+    Tile *pack_tiles = nullptr;      // the fused step's: 16-byte chunks, at most kPackThreads of them
+    int32_t n_pack_tiles = 0, pack_ctas = 0;
     int32_t batch_ctas = 0;
     int64_t *step_base = nullptr;    // two int64 in device memory: the step counter, then
                                      // the error flag of the staged sweep (an int32)
@@ -3606,6 +3395,7 @@ struct acf_batch {
     // launch geometry (tunable; results never depend on it)
     int block_threads = 256;
     int planes = 4;
+    bool planes_set = false;         // by set_launch
     int ctas_per_sm = 4;
     int staged_rows = 2;             // staged scheme: y rows per CTA
     int staged_stages = 0;           // staged scheme: ring buffers per CTA (0: automatic)
@@ -3706,6 +3496,7 @@ struct acf_batch {
     };
     std::vector<RoomAdjoint> badj;
     int64_t badj_capacity = 0, badj_recorded = 0, badj_step0 = 0;
+    void *badj_history = nullptr;    // device array of History<T>, one per room
     void *badj_table = nullptr;      // device array of AdjointParams<T>: 2 per room (the two copies of mu)
 
     size_t elem() const { return (size_t)precision; }
@@ -3809,13 +3600,36 @@ Room<T> make_room(const acf_batch *b, int r, const void *state = nullptr) {
     return s;
 }
 
+bool second_copies(const acf_batch *b) {
+    for (const RoomHost &h : b->rooms)
+        if (!h.second) return false;
+    return true;
+}
+
+// The second copies of p and v of the rooms that have none, zeroed on `st`; false when the device
+// has no room for one of them (those already there stay).
+bool make_second_copies(acf_batch *b, cudaStream_t st) {
+    for (RoomHost &h : b->rooms) {
+        if (h.second) continue;
+        const size_t bytes = ((size_t)4 * h.field + (size_t)h.pz) * b->elem();
+        if (dev_malloc(&h.second, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            h.second = nullptr;
+            return false;
+        }
+        b->room_table_dirty = true;
+        if (cudaMemsetAsync(h.second, 0, bytes, st) != cudaSuccess) return false;
+    }
+    return true;
+}
+
 template <typename T>
 int upload_room_table(acf_batch *b) {
     std::vector<Room<T>> table(b->rooms.size());
     for (size_t r = 0; r < b->rooms.size(); r++) table[r] = make_room<T>(b, (int)r);
     if (!b->room_table) ACF_CUDA(dev_malloc(&b->room_table, table.size() * sizeof(Room<T>)));
     ACF_CUDA(cudaMemcpy(b->room_table, table.data(), table.size() * sizeof(Room<T>), cudaMemcpyHostToDevice));
-    if (b->scheme == ACF_SCHEME_FUSED) {
+    if (second_copies(b)) {
         // Both parities: entry [parity * rooms + r] reads the copy that is current at that parity.
         const size_t n = b->rooms.size();
         std::vector<FusedParams<T>> fused(2 * n);
@@ -3842,35 +3656,69 @@ int upload_room_table(acf_batch *b) {
 }
 
 // Tiles in room order, then plane group, then (row, chunk) block: neighbouring tiles of one
-// room run close together, so the y- and x-neighbour rows they share are still in L2.
-int build_tiles(acf_batch *b) {
+// room run close together, so the y- and x-neighbour rows they share are still in L2. `width` z
+// elements per chunk, at most `threads` pairs per tile.
+int upload_tiles(const acf_batch *b, int width, int threads, int planes, Tile **to, int32_t *n_tiles,
+                 int32_t *ctas) {
     std::vector<Tile> tiles;
     for (size_t r = 0; r < b->rooms.size(); r++) {
         const RoomHost &h = b->rooms[r];
-        const int64_t nchunks = (h.nz + kVec - 1) / kVec;
+        const int64_t nchunks = (h.nz + width - 1) / width;
         const int64_t pairs = (int64_t)h.ny * nchunks;
-        for (int i0 = 0; i0 < h.nx; i0 += b->planes)
-            for (int64_t first = 0; first < pairs; first += b->block_threads) {
+        for (int i0 = 0; i0 < h.nx; i0 += planes)
+            for (int64_t first = 0; first < pairs; first += threads) {
                 Tile t{};
                 t.room = (int32_t)r;
                 t.first = (int32_t)first;
-                t.count = (int32_t)std::min<int64_t>(b->block_threads, pairs - first);
+                t.count = (int32_t)std::min<int64_t>(threads, pairs - first);
                 t.i_begin = i0;
-                t.i_end = std::min(h.nx, i0 + b->planes);
+                t.i_end = std::min(h.nx, i0 + planes);
                 tiles.push_back(t);
             }
     }
     if (tiles.size() > (size_t)INT32_MAX) return fail(ACF_ERR_ARGUMENT, "too many tiles");
-    dev_free(b->tiles);
-    b->tiles = nullptr;
-    ACF_CUDA(dev_malloc(&b->tiles, std::max<size_t>(1, tiles.size()) * sizeof(Tile)));
-    ACF_CUDA(cudaMemcpy(b->tiles, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice));
-    b->n_tiles = (int32_t)tiles.size();
+    dev_free(*to);
+    *to = nullptr;
+    ACF_CUDA(dev_malloc(to, std::max<size_t>(1, tiles.size()) * sizeof(Tile)));
+    ACF_CUDA(cudaMemcpy(*to, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice));
+    *n_tiles = (int32_t)tiles.size();
     // ctas_per_sm == 0: one CTA per tile, scheduled by the hardware; otherwise a persistent
     // grid of ctas_per_sm CTAs per SM striding over the table.
-    b->batch_ctas = b->ctas_per_sm == 0 ? std::max(1, b->n_tiles)
-                                        : std::max(1, std::min(b->n_tiles, b->ctas_per_sm * b->sms));
+    *ctas = b->ctas_per_sm == 0 ? std::max(1, *n_tiles)
+                                : std::max(1, std::min(*n_tiles, b->ctas_per_sm * b->sms));
     return ACF_OK;
+}
+
+// Planes per tile of the fused batch step, unless set_launch named them: of 4 to 8 the number with
+// the shortest run of whole waves, each as long as its planes and 1.5 more for a tile's prologue. us
+// per step at 4, 5, 6 and 8 planes in single precision with air (waves): 4 rooms of 60 to 110 43, 48,
+// 53, 44 (1.8, 1.5, 1.2, 0.95); 3 of 96 to 160 89, 89, 94, 95 (4.7, 3.8, 3.2, 2.4); 8 of 60 to 200
+// 156, 154, 155, 159; in double precision 279, 274, 272, 271 (21, 17, 14, 11).
+int pack_planes(const acf_batch *b) {
+    if (b->planes_set) return b->planes;
+    const int width = 16 / (int)b->elem();
+    const int64_t slots = (int64_t)b->sms * pack_batch_blocks((int)b->elem(), b->n_relax > 0, false);
+    int best = 8;
+    double best_cost = 0.0;
+    for (int planes = 8; planes >= 4; planes--) {
+        int64_t tiles = 0;
+        for (const RoomHost &h : b->rooms)
+            tiles += (h.nx + planes - 1) / planes *
+                     (((int64_t)h.ny * ((h.nz + width - 1) / width) + kPackThreads - 1) / kPackThreads);
+        const double cost = (double)((tiles + slots - 1) / slots) * (planes + 1.5);
+        if (planes == 8 || cost < best_cost) {
+            best = planes;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+int build_tiles(acf_batch *b) {
+    int rc = upload_tiles(b, kVec, b->block_threads, b->planes, &b->tiles, &b->n_tiles, &b->batch_ctas);
+    if (rc) return rc;
+    return upload_tiles(b, 16 / (int)b->elem(), std::min(b->block_threads, kPackThreads), pack_planes(b),
+                        &b->pack_tiles, &b->n_pack_tiles, &b->pack_ctas);
 }
 
 struct LaunchShape {
@@ -3959,13 +3807,6 @@ void fill_pairs(float2 *pairs, const RoomHost &h) {
         put_neg(kPairNegMean + r, h.mean[r]);
     }
 }
-
-template <typename T, bool L, bool W, int NR>
-struct BatchFused {
-    static void launch(const FusedBatchParams<T> &p, dim3 g, dim3 b, cudaStream_t st) {
-        fused_batch<T, L, W, NR><<<g, b, 0, st>>>(p);
-    }
-};
 
 // Ring layout and shared memory of the staged sweep for `rows` y rows per CTA.
 struct StagedLayout {
@@ -4142,22 +3983,25 @@ void launch_pair(acf_batch *b, int32_t local, bool back, cudaStream_t st) {
     b->launches += 1;
 }
 
+// The fused step of a batch from the copy all rooms are at.
+template <typename T>
+FusedBatchParams<T> fused_batch_params(const acf_batch *b, int32_t local) {
+    FusedBatchParams<T> p{};
+    p.rooms = (const FusedParams<T> *)b->fused_table + (b->rooms[0].cur ? b->rooms.size() : 0);
+    p.tiles = b->pack_tiles;
+    p.n_tiles = b->n_pack_tiles;
+    p.local_step = local;
+    p.step_base = b->step_base;
+    return p;
+}
+
 // Launch one step; the fused scheme flips the room's current buffer, as the kernel will have
 // done by the time anything queued after it runs.
 template <typename T>
 void launch_step(acf_batch *b, int32_t local, cudaStream_t st, cudaEvent_t *events) {
     if (events) cudaEventRecord(events[0], st);
     if (b->rooms.size() > 1 && b->fused()) {
-        // The tile-table launch keeps the generic column: the lean column there measured 82-89
-        // Gcell-updates/s on the 64 uneven rooms against 94 (its registers cost warps per SM).
-        const dim3 grid(b->batch_ctas), block(b->block_threads);
-        FusedBatchParams<T> p{};
-        p.rooms = (const FusedParams<T> *)b->fused_table + (b->rooms[0].cur ? b->rooms.size() : 0);
-        p.tiles = b->tiles;
-        p.n_tiles = b->n_tiles;
-        p.local_step = local;
-        p.step_base = b->step_base;
-        dispatch_pressure<T, BatchFused>(b->any_layer, b->any_walls, b->n_relax, p, grid, block, st);
+        launch_pack_batch(fused_batch_params<T>(b, local), b->any_layer, b->any_walls, b->n_relax, b->pack_ctas, st);
         for (RoomHost &h : b->rooms) h.cur ^= 1;
         if (events) {
             cudaEventRecord(events[1], st);
@@ -4367,13 +4211,11 @@ bool one_sweep_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
         if (!h.second) {
             const size_t bytes = ((size_t)4 * h.field + (size_t)h.pz) * b->elem();
             size_t free_bytes = 0, total_bytes = 0;
-            if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess || bytes > free_bytes / 16 ||
-                dev_malloc(&h.second, bytes) != cudaSuccess) {
+            if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess || bytes > free_bytes / 16) {
                 cudaGetLastError();
-                h.second = nullptr;
                 return false;
             }
-            if (cudaMemsetAsync(h.second, 0, bytes, st) != cudaSuccess) return false;
+            if (!make_second_copies(b, st)) return false;
         }
         b->one_sweep_state = 1;
     }
@@ -4629,6 +4471,7 @@ void free_batch(acf_batch *b) {
         dev_free(ra.grad_src);
     }
     dev_free(b->badj_table);
+    dev_free(b->badj_history);
     dev_free(b->pair_ring);
     dev_free(b->pair_progress);
     dev_free(b->psi2);
@@ -4638,6 +4481,7 @@ void free_batch(acf_batch *b) {
     dev_free(b->room_table);
     dev_free(b->fused_table);
     dev_free(b->tiles);
+    dev_free(b->pack_tiles);
     dev_free(b->step_base);
     dev_free(b->energy_scratch);
     delete b;
@@ -4783,7 +4627,8 @@ int create_batch(int32_t n_rooms, const acf_config *configs, acf_batch *b) {
         return fail(ACF_ERR_MEMORY, "cudaMalloc of energy scratch failed");
     if (batched) {
         // one CTA per tile of 128 (row, chunk) pairs x 8 planes: the best measured schedule on
-        // uneven-room batches (persistent grids lose to the hardware scheduler here)
+        // uneven-room batches (persistent grids lose to the hardware scheduler here); the fused
+        // step's tiles choose their own planes (pack_planes)
         b->block_threads = 128;
         b->planes = 8;
         b->ctas_per_sm = 0;
@@ -5311,9 +5156,11 @@ int set_launch(acf_batch *b, int32_t block_threads, int32_t planes, int32_t ctas
     if (b->rooms.size() == 1 && (b->rooms[0].nx + planes - 1) / planes > 65535)
         return fail(ACF_ERR_ARGUMENT, "nx / planes exceeds the 65535 grid limit; use more planes per block");
     DeviceGuard guard(b->device);
-    const bool changed = block_threads != b->block_threads || planes != b->planes || ctas_per_sm != b->ctas_per_sm;
+    const bool changed = block_threads != b->block_threads || planes != b->planes || ctas_per_sm != b->ctas_per_sm ||
+                         !b->planes_set;
     b->block_threads = block_threads;
     b->planes = planes;
+    b->planes_set = true;
     b->ctas_per_sm = ctas_per_sm;
     if (changed) {
         b->graph_dirty = b->adj_graphs_dirty = true;
@@ -5588,14 +5435,14 @@ constexpr int64_t kAdjointChunk = 64;
 // the history in `hist`. Receivers record only when `receivers` is set, so a recompute leaves
 // the caller's recordings alone. With `checkpoints`, the state at every multiple of the
 // checkpoint interval (counted from the recorded run's first step) is copied out first. With
-// `lean` (single precision, nz a multiple of 4, the room's own fields current in its primary
-// copy, no D/psi history) each step is one lean step into the other copy, flipping the current
-// copy as the fused scheme does; graphs hold an even number of steps, so a replay leaves it as
-// it found it.
+// `one_sweep` (the room's own fields, current in its primary copy, no checkpoints) each step is
+// one fused step into the other copy, flipping the current copy as the fused scheme does; graphs
+// hold an even number of steps, so a replay leaves it as it found it. Without it (a recompute,
+// runs with checkpoints, or no memory for the second copy) each step is the two sweeps.
 template <typename T>
 int record_steps(acf_batch *b, acf_batch::Graph &g, const void *state, const History<T> &hist,
                  int64_t s0, int64_t n, bool receivers, cudaStream_t st, bool checkpoints,
-                 bool lean = false) {
+                 bool one_sweep = false) {
     const RoomHost &h = b->rooms[0];
     StepParams<T> p{};
     p.room = make_room<T>(b, 0, state);
@@ -5604,27 +5451,34 @@ int record_steps(acf_batch *b, acf_batch::Graph &g, const void *state, const His
     p.step_base = b->step_base;
     p.planes = b->planes;
     const LaunchShape L = single_shape(b);
-    const int per_step = lean ? 1 : 2;
+    const int per_step = one_sweep ? 1 : 2;
     auto launch = [&](int32_t local, cudaStream_t s) {
-        if constexpr (sizeof(T) == 4) {
-            if (lean) {
-                RoomHost &hr = b->rooms[0];
-                LeanRecParams q{};
-                q.g.f.room = make_room<float>(b, 0);
-                q.g.f.np = (float *)b->other_ptr(0, ACF_FIELD_P);
-                q.g.f.nvx = (float *)b->other_ptr(0, ACF_FIELD_VX);
-                q.g.f.nvy = (float *)b->other_ptr(0, ACF_FIELD_VY);
-                q.g.f.nvz = (float *)b->other_ptr(0, ACF_FIELD_VZ);
-                q.g.f.step_base = b->step_base;
-                q.g.f.local_step = local;
-                q.g.f.planes = b->planes;
-                fill_pairs(q.g.pairs, hr);
-                q.hist = hist;
-                dispatch_pressure<float, LeanRecStep>(hr.has_layer, hr.has_walls, hr.n_relax, q, L.grid,
-                                                      L.block, s);
-                hr.cur ^= 1;
-                return;
+        if (one_sweep) {
+            RoomHost &hr = b->rooms[0];
+            FusedParams<T> f{};
+            f.room = make_room<T>(b, 0);
+            f.np = (T *)b->other_ptr(0, ACF_FIELD_P);
+            f.nvx = (T *)b->other_ptr(0, ACF_FIELD_VX);
+            f.nvy = (T *)b->other_ptr(0, ACF_FIELD_VY);
+            f.nvz = (T *)b->other_ptr(0, ACF_FIELD_VZ);
+            f.step_base = b->step_base;
+            f.local_step = local;
+            f.planes = b->planes;
+            bool lean = false;
+            if constexpr (sizeof(T) == 4) {
+                lean = hr.nz % kVec == 0 && !hist.fields;
+                if (lean) {
+                    LeanRecParams q{};
+                    q.g.f = f;
+                    fill_pairs(q.g.pairs, hr);
+                    q.hist = hist;
+                    dispatch_pressure<float, LeanRecStep>(hr.has_layer, hr.has_walls, hr.n_relax, q, L.grid,
+                                                          L.block, s);
+                }
             }
+            if (!lean) launch_pack_rec(f, hist, hr.has_layer, hr.has_walls, hr.n_relax, b->block_threads, s);
+            hr.cur ^= 1;
+            return;
         }
         StepParams<T> q = p;
         q.local_step = local;
@@ -5678,31 +5532,19 @@ int forward_record_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cuda
         hist.fields_step0 = step_offset;
         hist.fields_slots = A.every;
     }
-    // Without air the history is the boundary shell alone, which the lean single-precision step
-    // writes as it goes: one sweep per recorded step instead of two, into the second copy of p
-    // and v (allocated here when the solver's scheme has none; two sweeps if that fails).
-    bool lean = !air && sizeof(T) == 4 && b->rooms.size() == 1 && b->rooms[0].nz % kVec == 0 &&
-                b->rooms[0].cur == 0;
-    if (lean && !b->rooms[0].second) {
-        RoomHost &h = b->rooms[0];
-        const size_t bytes = ((size_t)4 * h.field + (size_t)h.pz) * b->elem();
-        if (dev_malloc(&h.second, bytes) != cudaSuccess) {
-            cudaGetLastError();
-            h.second = nullptr;
-            lean = false;
-        } else {
-            ACF_CUDA(cudaMemsetAsync(h.second, 0, bytes, st));
-        }
-    }
-    const int mode = A.fields_recorded ? 1 : (lean ? 2 : 0);
+    // One fused step per recorded step instead of two sweeps, into the second copy of p and v
+    // (allocated here when the solver's scheme has none; two sweeps if that fails). Checkpoints
+    // are copied from the primary copy at any step, so a run that keeps them stays in place.
+    const bool one_sweep = (!air || A.fields_recorded) && b->rooms[0].cur == 0 && make_second_copies(b, st);
+    const int mode = (A.fields_recorded ? 1 : 0) + (one_sweep ? 2 : 0);
     if (mode != A.direct_mode) {
         b->adj_graphs_dirty = true;           // the record graph holds the history pointers
         A.direct_mode = mode;
     }
     int rc = record_steps<T>(b, b->g_record, b->field_ptr(0, ACF_FIELD_P), hist, step_offset, n_steps,
-                             true, st, air && !A.fields_recorded, lean);
+                             true, st, air && !A.fields_recorded, one_sweep);
     if (rc) return rc;
-    if (lean) {   // an odd number of steps ends in the second copy: bring the state back
+    if (one_sweep) {   // an odd number of steps ends in the second copy: bring the state back
         rc = make_primary(b, st);
         if (rc) return rc;
     }
@@ -5946,11 +5788,12 @@ int adjoint_prepare(acf_batch *b, int32_t flags, int64_t max_steps, int32_t ever
         const RoomHost &h = b->rooms[0];
         const double whole = (double)max_steps * (1 + h.n_relax) * h.field * b->elem();
         size_t free_bytes = 0, total_bytes = 0;
-        {
-            std::lock_guard<std::mutex> hold(block_cache().lock);
-            block_cache().trim(0);
-        }
         ACF_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+        {                          // idle blocks of the cache are given back before an allocation fails
+            std::lock_guard<std::mutex> hold(block_cache().lock);
+            for (const BlockCache::Block &idle : block_cache().idle)
+                if (idle.device == b->device) free_bytes += idle.bytes;
+        }
         every = whole <= 0.6 * (double)free_bytes ? (int32_t)std::min<int64_t>(max_steps, INT32_MAX)
                                                    : (int32_t)std::ceil(std::sqrt((double)max_steps));
     }
@@ -6172,6 +6015,10 @@ int upload_adjoint_table(acf_batch *b, int64_t n) {
         o.out_d = a.ld;
         (void)n;
     }
+    std::vector<History<T>> history(nr);
+    for (size_t r = 0; r < nr; r++) history[r] = table[r].hist;
+    if (!b->badj_history) ACF_CUDA(dev_malloc(&b->badj_history, nr * sizeof(History<T>)));
+    ACF_CUDA(cudaMemcpy(b->badj_history, history.data(), nr * sizeof(History<T>), cudaMemcpyHostToDevice));
     if (!b->badj_table) ACF_CUDA(dev_malloc(&b->badj_table, table.size() * sizeof(AdjointParams<T>)));
     ACF_CUDA(cudaMemcpy(b->badj_table, table.data(), table.size() * sizeof(AdjointParams<T>),
                         cudaMemcpyHostToDevice));
@@ -6188,6 +6035,23 @@ int batch_forward_record_impl(acf_batch *b, int64_t n_steps, int64_t step_offset
     }
     int rc = upload_adjoint_table<T>(b, n_steps);
     if (rc) return rc;
+    // Fused steps between the two copies of p and v; on the two-sweep scheme an odd last step is
+    // the sweeps, in place, so that the state is in the rooms' own copies before and after. All
+    // of them are the sweeps where the device has no room for second copies.
+    const bool one_sweep = make_second_copies(b, st);
+    if (one_sweep && b->room_table_dirty) {
+        rc = upload_room_table<T>(b);
+        if (rc) return rc;
+    }
+    const bool alternating = b->scheme == ACF_SCHEME_FUSED;
+    const int64_t fused_steps = !one_sweep ? 0 : alternating ? n_steps : n_steps / 2 * 2;
+    set_step_base<<<1, 1, 0, st>>>(b->step_base, step_offset);
+    for (int64_t t = 0; t < fused_steps; t++) {
+        FusedBatchParams<T> p = fused_batch_params<T>(b, (int32_t)t);
+        p.history = (const History<T> *)b->badj_history;
+        launch_pack_batch(p, b->any_layer, b->any_walls, b->n_relax, b->pack_ctas, st);
+        for (RoomHost &h : b->rooms) h.cur ^= 1;
+    }
     BatchParams<T> v{};
     v.rooms = (const Room<T> *)b->room_table;
     v.tiles = b->tiles;
@@ -6199,14 +6063,13 @@ int batch_forward_record_impl(acf_batch *b, int64_t n_steps, int64_t step_offset
     p.n_tiles = b->n_tiles;
     p.step_base = b->step_base;
     const dim3 grid(b->batch_ctas), block(b->block_threads);
-    set_step_base<<<1, 1, 0, st>>>(b->step_base, step_offset);
-    for (int64_t t = 0; t < n_steps; t++) {
+    for (int64_t t = fused_steps; t < n_steps; t++) {
         v.local_step = p.local_step = (int32_t)t;
         if (b->any_layer) velocity_batch<T, true><<<grid, block, 0, st>>>(v);
         else velocity_batch<T, false><<<grid, block, 0, st>>>(v);
         dispatch_pressure<T, BatchRecPressure>(b->any_layer, b->any_walls, b->n_relax, p, grid, block, st);
     }
-    b->launches += 2 * n_steps + 1;
+    b->launches += 2 * n_steps - fused_steps + 1;
     ACF_CUDA(cudaGetLastError());
     return ACF_OK;
 }

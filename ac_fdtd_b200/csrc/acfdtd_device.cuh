@@ -178,6 +178,23 @@ struct FusedParams {
     int32_t planes;
 };
 
+// One unit of work of a batched sweep: up to blockDim.x consecutive (row, chunk) pairs of one
+// room, over the x planes [i_begin, i_end).
+struct Tile {
+    int32_t room, first, count, i_begin, i_end, reserved;
+};
+
+// One fused step of every room: rooms points at the descriptions for the copy all rooms are at.
+template <typename T>
+struct FusedBatchParams {
+    const FusedParams<T> *rooms;
+    const Tile *tiles;
+    int32_t n_tiles;
+    int32_t local_step;
+    const int64_t *step_base;
+    const History<T> *history;     // recorded runs: one per room
+};
+
 // ------------------------------------------------------------------------------------------
 // Walls, sources and receivers of one (row, chunk) column.
 
@@ -309,9 +326,9 @@ __device__ __forceinline__ void record_receivers(const Room<T> &s, uint32_t mask
 // row-major over that face's two other axes. A column on an x-face plane or a y-face row owns
 // contiguous entries for its whole chunk; elsewhere only its k = 0 and k = nz - 1 cells are on a
 // (z) face.
-template <typename T>
+template <typename T, int W = kVec>
 __device__ __forceinline__ void record_shell(const Room<T> &s, const History<T> &hist, int i, int j,
-                                             int k0, int64_t step, const T P[kVec], const T PT[kVec]) {
+                                             int k0, int64_t step, const T (&P)[W], const T (&PT)[W]) {
     const int64_t slot = step - hist.shell_step0;
     if (slot < 0 || slot >= hist.shell_steps) return;
     T *hp = hist.shell + slot * 2 * hist.shell_total;
@@ -321,7 +338,7 @@ __device__ __forceinline__ void record_shell(const Room<T> &s, const History<T> 
         const int f = x_face ? (i == 0 ? 0 : 1) : (j == 0 ? 2 : 3);
         const int64_t at = hist.face_off[f] + (x_face ? (int64_t)j : (int64_t)i) * s.nz + k0;
 #pragma unroll
-        for (int e = 0; e < kVec; e++)
+        for (int e = 0; e < W; e++)
             if (k0 + e < s.nz) {
                 hp[at + e] = P[e];
                 ht[at + e] = PT[e];
@@ -334,9 +351,9 @@ __device__ __forceinline__ void record_shell(const Room<T> &s, const History<T> 
         ht[hist.face_off[4] + at] = PT[0];
     }
     const int top = s.nz - 1 - k0;   // element of k = nz - 1, unless that cell is also k = 0
-    if (s.nz > 1 && top >= 0 && top < kVec) {
+    if (s.nz > 1 && top >= 0 && top < W) {
 #pragma unroll
-        for (int e = 0; e < kVec; e++)
+        for (int e = 0; e < W; e++)
             if (e == top) {
                 hp[hist.face_off[5] + at] = P[e];
                 ht[hist.face_off[5] + at] = PT[e];

@@ -1,34 +1,29 @@
-// acfdtd_fused64.cu -- the fused step in double precision.
+// acfdtd_fused_kernel.cuh -- the fused step of one column of 16-byte chunks, in either precision.
 //
-// Bound by HBM: (8 + 2R) elements per cell and step, 112 bytes with three relaxation states. The step
-// with four z elements per thread held its loads in 128 registers, so an SM had 16 warps and the
-// rest of the loads of a plane waited for them: 0.69 of the measured copy rate on 251 x 240 x 263
-// with every term, no better than the two sweeps (397 against 404 us, which move 144 bytes). Here a
-// thread takes two elements, one 16-byte access per field, so that twice the warps are resident with
-// the same bytes in flight each; faces on walls are not asked for (the pressure outside is the
-// cell's own, a difference of zero), and layer factors that are exactly 1 are skipped.
-// Measured (us per step; TB/s of the 112 or 64 bytes per cell): 251 x 240 x 263 with every term 397 to
-// 294 (6.04), walls only 214 to 161 (6.31); 320^3 with every term 589 (6.23, 0.96 of the copy);
-// 160 x 161 x 163 128 to 87. Four planes per block: 8 cost 2 to 8 % more, 16 up to 30 %.
+// Faces on walls are not asked for (the pressure outside is the cell's own, a difference of zero:
+// neighbour offsets are 0 where the room ends, so no load is conditional), layer factors that are
+// exactly 1 are skipped, and a chunk that reaches past nz repeats its last real pressure.
 
-#include "acfdtd_fused64.cuh"
-
-#include <algorithm>
+#ifndef ACFDTD_FUSED_KERNEL_CUH
+#define ACFDTD_FUSED_KERNEL_CUH
 
 #include "acfdtd_pack.cuh"
 
 namespace acf {
 namespace {
 
-template <typename T>
-__device__ __forceinline__ Pack<T> pack_ldg(const T *a) {
+__device__ __forceinline__ Pack<double> pack_ldg(const double *a) {
     return {__ldg(reinterpret_cast<const double2 *>(a))};
 }
+__device__ __forceinline__ Pack<float> pack_ldg(const float *a) {
+    const float4 v = __ldg(reinterpret_cast<const float4 *>(a));
+    return {lo2(v), hi2(v)};
+}
 
-template <bool LAYER, bool WALLS, int NR>
-__device__ __forceinline__ void pack_column(const FusedParams<double> &f, int i_begin, int i_end, int j, int c,
-                                            int64_t step) {
-    using T = double;
+// One column of chunks over planes [i_begin, i_end). REC: also write the forward history.
+template <typename T, bool LAYER, bool WALLS, int NR, bool REC = false>
+__device__ __forceinline__ void pack_column(const FusedParams<T> &f, int i_begin, int i_end, int j, int c,
+                                            int64_t step, const History<T> *hist = nullptr) {
     using P = Pack<T>;
     constexpr int W = P::W;
     const Room<T> &s = f.room;
@@ -43,28 +38,31 @@ __device__ __forceinline__ void pack_column(const FusedParams<double> &f, int i_
     bool all_points = false;
     const uint32_t points = (s.n_src | s.n_rec) != 0 ? column_points(s, j, k0, all_points, W) : 0u;
     const bool any_mine = points != 0 || all_points;
-    const bool wall_column = WALLS && (j == 0 || j + 1 == s.ny || k0 == 0 || k0 + W >= s.nz);
+    const bool wall_column = (WALLS || REC) && (j == 0 || j + 1 == s.ny || k0 == 0 || k0 + W >= s.nz);
 
-    T fy_c = 1.0, fy_l = 1.0, fy_h = 1.0;
+    T fy_c = T(1), fy_l = T(1), fy_h = T(1);
     bool damp_y = false, damp_z = false;
     if (LAYER) {
         fy_c = __ldg(s.cell[1] + j);
         fy_l = __ldg(s.face[1] + j);
         fy_h = __ldg(s.face[1] + j + 1);
-        damp_y = fy_c != 1.0 || fy_l != 1.0 || fy_h != 1.0;
+        damp_y = fy_c != T(1) || fy_l != T(1) || fy_h != T(1);
 #pragma unroll
         for (int e = 0; e <= W; e++) {
-            damp_z = damp_z || __ldg(s.face[2] + min(k0 + e, s.nz)) != 1.0;
-            if (e < W) damp_z = damp_z || __ldg(s.cell[2] + min(k0 + e, s.nz - 1)) != 1.0;
+            damp_z = damp_z || __ldg(s.face[2] + min(k0 + e, s.nz)) != T(1);
+            if (e < W) damp_z = damp_z || __ldg(s.cell[2] + min(k0 + e, s.nz - 1)) != T(1);
         }
     }
     // z factors at cells and at faces, read where used (they stay in L1)
-    auto z_cells = [&](const P &v) {
-        return P{make_double2(v.a.x * __ldg(s.cell[2] + k0), v.a.y * __ldg(s.cell[2] + min(k0 + 1, s.nz - 1)))};
+    auto z_times = [&](const P &v, const T *profile, int last) {
+        T x[W];
+        unpack(v, x);
+#pragma unroll
+        for (int e = 0; e < W; e++) x[e] = x[e] * __ldg(profile + min(k0 + e, last));
+        return repack(x);
     };
-    auto z_faces = [&](const P &v) {
-        return P{make_double2(v.a.x * __ldg(s.face[2] + k0), v.a.y * __ldg(s.face[2] + k0 + 1))};
-    };
+    auto z_cells = [&](const P &v) { return z_times(v, s.cell[2], s.nz - 1); };
+    auto z_faces = [&](const P &v) { return z_times(v, s.face[2], s.nz); };
     auto moved = [&](const P &v, const P &high, const P &low) { return psub(v, pmul(psub(high, low), cv)); };
 
     // Carried from plane to plane: p(i) and the updated vx on face i.
@@ -77,12 +75,12 @@ __device__ __forceinline__ void pack_column(const FusedParams<double> &f, int i_
         if (tail) pc = mirrored(pc, real);
         if (LAYER) {
             const T fx = __ldg(s.face[0] + i_begin);
-            if (fx != 1.0) xl = pmul(xl, fx);
+            if (fx != T(1)) xl = pmul(xl, fx);
             if (damp_y) xl = pmul(xl, fy_c);
             if (damp_z) xl = z_cells(xl);
         }
     }
-    T bad = finite_start(0.0);
+    auto bad = finite_start(T(0));
 
     for (int i = i_begin; i < i_end; i++) {
         const int64_t base = (int64_t)i * s.plane + column;
@@ -102,7 +100,7 @@ __device__ __forceinline__ void pack_column(const FusedParams<double> &f, int i_
         P xh = pack_ldg(s.vx + base + s.plane), yl = pack_ldg(s.vy + base), yh = pack_ldg(s.vy + base + s.pz);
         P zl = pack_ldg(s.vz + base);
         const T pz_l = __ldg(s.p + base + z_lo), pz_h = __ldg(s.p + base + z_hi);
-        T za = k0 + W <= s.nz ? __ldg(s.vz + base + W) : 0.0;
+        T za = k0 + W <= s.nz ? __ldg(s.vz + base + W) : T(0);
         P S[NR > 0 ? NR : 1];
 #pragma unroll
         for (int r = 0; r < NR; r++) S[r] = pload(s.psi + r * s.field + base);
@@ -113,12 +111,12 @@ __device__ __forceinline__ void pack_column(const FusedParams<double> &f, int i_
         yl = moved(yl, pc, py_l);
         yh = moved(yh, py_h, pc);
         zl = moved(zl, pc, below_of(pc, pz_l));
-        za = za - cv * ((z_hi == W ? pz_h : pc.a.y) - pc.a.y);
-        T fx = 1.0;
+        za = za - cv * ((z_hi == W ? pz_h : last_of(pc)) - last_of(pc));
+        T fx = T(1);
         if (LAYER) {   // x, y, z order; an axis whose factors here are all exactly 1 is skipped
             fx = __ldg(s.cell[0] + i);
             const T fx_h = __ldg(s.face[0] + i + 1);
-            if (fx != 1.0 || fx_h != 1.0) {
+            if (fx != T(1) || fx_h != T(1)) {
                 xh = pmul(xh, fx_h);
                 yl = pmul(yl, fx);
                 yh = pmul(yh, fx);
@@ -144,31 +142,41 @@ __device__ __forceinline__ void pack_column(const FusedParams<double> &f, int i_
         P d = psub(xh, xl);
         d = padd(d, psub(yh, yl));
         d = padd(d, psub(above_of(zl, za), zl));
+        if (REC && hist->fields) {               // D and psi of this step, for the air gradients
+            const int64_t rel = step - hist->fields_step0;
+            if (rel >= 0) {
+                T *h = hist->fields + rel % hist->fields_slots * (1 + NR) * s.field + base;
+                pstore_streaming(h, d);
+#pragma unroll
+                for (int r = 0; r < NR; r++) pstore_streaming(h + (1 + r) * s.field, S[r]);
+            }
+        }
         P pe = pc;
 #pragma unroll
         for (int r = 0; r < NR; r++) {
             const P target = pmul(d, s.gain[r]);
             const P offset = psub(S[r], target);
-            P next = padd(pmul(offset, s.decay[r]), target);
-            pe = padd(pe, pmul(offset, s.mean[r]));
+            P next = psub(target, pmul(offset, -s.decay[r]));     // see padd
+            pe = psub(pe, pmul(offset, -s.mean[r]));
             if (tail) next = keep_from(next, S[r], real);
             S[r] = next;
         }
-        if (NR > 0) pe = padd(pe, pmul(d, s.relax_scale));
+        if (NR > 0) pe = psub(pe, pmul(d, -s.relax_scale));
         pe = psub(pe, pmul(d, s.cp));
-        if (wall_column || (WALLS && (i == 0 || !inner))) {
+        if (wall_column || ((WALLS || REC) && (i == 0 || !inner))) {
             T pn[W], po[W];
             unpack(pe, pn);
             unpack(pc, po);
+            if (REC && hist->shell) record_shell<T, W>(s, *hist, i, j, k0, step, po, pn);
 #pragma unroll
             for (int e = 0; e < W; e++) {
                 T fu, fp;
-                if (e < real && wall_pair(s, i, j, k0 + e, fu, fp)) pn[e] = pn[e] * fu - po[e] * fp;
+                if (WALLS && e < real && wall_pair(s, i, j, k0 + e, fu, fp)) pn[e] = pn[e] * fu - po[e] * fp;
             }
             pe = repack(pn);
         }
         if (LAYER) {
-            if (fx != 1.0) pe = pmul(pe, fx);
+            if (fx != T(1)) pe = pmul(pe, fx);
             if (damp_y) pe = pmul(pe, fy_c);
             if (damp_z) pe = z_cells(pe);
         }
@@ -199,45 +207,7 @@ __device__ __forceinline__ void pack_column(const FusedParams<double> &f, int i_
     report_nonfinite(s.status, is_bad(bad));
 }
 
-template <bool LAYER, bool WALLS, int NR>
-__global__ void __launch_bounds__(128, NR > 0 ? 6 : 8) pack_sweep(const __grid_constant__ FusedParams<double> f) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (c * Pack<double>::W >= f.room.nz || j >= f.room.ny) return;
-    const bool any_point = (f.room.n_src | f.room.n_rec) != 0;
-    const int64_t step = any_point ? (*f.step_base + f.local_step) : 0;
-    const int i_begin = blockIdx.z * f.planes;
-    pack_column<LAYER, WALLS, NR>(f, i_begin, min(f.room.nx, i_begin + f.planes), j, c, step);
-}
-
-template <bool LAYER, bool WALLS>
-void launch_pack(const FusedParams<double> &f, int n_relax, dim3 grid, dim3 block, cudaStream_t st) {
-    switch (n_relax) {
-        case 0: pack_sweep<LAYER, WALLS, 0><<<grid, block, 0, st>>>(f); break;
-        case 1: pack_sweep<LAYER, WALLS, 1><<<grid, block, 0, st>>>(f); break;
-        case 2: pack_sweep<LAYER, WALLS, 2><<<grid, block, 0, st>>>(f); break;
-        case 3: pack_sweep<LAYER, WALLS, 3><<<grid, block, 0, st>>>(f); break;
-        default: pack_sweep<LAYER, WALLS, 4><<<grid, block, 0, st>>>(f); break;
-    }
-}
-
 }  // namespace
-
-void launch_pack_sweep(const FusedParams<double> &f, bool layer, bool walls, int n_relax, int block_threads,
-                       cudaStream_t st) {
-    const int chunks = (f.room.nz + Pack<double>::W - 1) / Pack<double>::W;
-    int bx = 1;
-    while (bx < chunks && bx < 32) bx <<= 1;
-    const int by = std::max(1, std::min<int>(f.room.ny, std::min(block_threads, 128) / bx));
-    const dim3 block(bx, by, 1);
-    const dim3 grid((chunks + bx - 1) / bx, (f.room.ny + by - 1) / by, (f.room.nx + f.planes - 1) / f.planes);
-    if (layer) {
-        if (walls) launch_pack<true, true>(f, n_relax, grid, block, st);
-        else launch_pack<true, false>(f, n_relax, grid, block, st);
-    } else {
-        if (walls) launch_pack<false, true>(f, n_relax, grid, block, st);
-        else launch_pack<false, false>(f, n_relax, grid, block, st);
-    }
-}
-
 }  // namespace acf
+
+#endif

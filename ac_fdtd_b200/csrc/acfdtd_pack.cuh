@@ -34,6 +34,13 @@ __device__ __forceinline__ void pstore(float *x, const Pack<float> &v) {
 }
 __device__ __forceinline__ void pstore(double *x, const Pack<double> &v) { *reinterpret_cast<double2 *>(x) = v.a; }
 
+__device__ __forceinline__ void pstore_streaming(float *x, const Pack<float> &v) {
+    __stcs(reinterpret_cast<float4 *>(x), make_float4(v.a.x, v.a.y, v.b.x, v.b.y));
+}
+__device__ __forceinline__ void pstore_streaming(double *x, const Pack<double> &v) {
+    __stcs(reinterpret_cast<double2 *>(x), v.a);
+}
+
 // Sums: in padd y is never a product (see add2); "plus a product" is psub of the product by the
 // negated coefficient.
 __device__ __forceinline__ Pack<float> psub(const Pack<float> &x, const Pack<float> &y) {
