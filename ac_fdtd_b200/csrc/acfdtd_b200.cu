@@ -4083,7 +4083,7 @@ void launch_step(acf_batch *b, int32_t local, cudaStream_t st, cudaEvent_t *even
                     dispatch_pressure<float, LeanStepPadded>(h.has_layer, h.has_walls, h.n_relax, g, L.grid,
                                                              L.block, st);
             } else {
-                launch_pack_sweep(f, h.has_layer, h.has_walls, h.n_relax, b->block_threads, st);
+                launch_pack_sweep(f, h.has_layer, h.has_walls, h.n_relax, b->block_threads, true, st);
             }
         }
         h.cur ^= 1;
@@ -4926,7 +4926,8 @@ void fused_slab_step(acf_batch *const *parts, int n, const int32_t *own_lo, cons
                 dispatch_pressure<float, LeanStepPadded>(h.has_layer, h.has_walls, h.n_relax, lp, L.grid,
                                                          L.block, streams[q]);
         } else {
-            launch_pack_sweep(f[q], h.has_layer, h.has_walls, h.n_relax, parts[q]->block_threads, streams[q]);
+            launch_pack_sweep(f[q], h.has_layer, h.has_walls, h.n_relax, parts[q]->block_threads, false,
+                              streams[q]);
         }
         parts[q]->launches += 1;
         after(q);

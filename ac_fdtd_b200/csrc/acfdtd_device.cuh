@@ -78,6 +78,18 @@ __device__ __forceinline__ void store_streaming(double *a, const double v[4]) {
     __stcs(reinterpret_cast<double2 *>(a + 2), make_double2(v[2], v[3]));
 }
 
+// The start of a kernel that launch_after may have launched before the kernel in front of it
+// has finished (programmatic dependent launch). Every thread passes the wait before it reads anything
+// a kernel writes, or writes: it ends when that kernel is complete and its writes are visible. The
+// first instruction lets the next step's blocks be launched as soon as all of this kernel's have started,
+// into the room that its last blocks leave.
+__device__ __forceinline__ void step_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void step_begin() {
+    step_next();
+    step_wait();
+}
+
 // Ask L2 for the line holding `a` ahead of its load: the request holds no register and no
 // shared memory, so a marching thread can have its next plane on the way from DRAM while it
 // computes the current one. Only addresses the thread will load later are passed.

@@ -16,12 +16,14 @@
 #include <algorithm>
 
 #include "acfdtd_fused_kernel.cuh"
+#include "acfdtd_host.cuh"
 
 namespace acf {
 namespace {
 
 template <bool LAYER, bool WALLS, int NR>
 __global__ void __launch_bounds__(128, NR > 0 ? 6 : 8) pack_sweep(const __grid_constant__ FusedParams<double> f) {
+    step_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (c * Pack<double>::W >= f.room.nz || j >= f.room.ny) return;
@@ -39,6 +41,7 @@ struct RecordParams {
 
 template <typename T, bool LAYER, bool WALLS, int NR>
 __global__ void __launch_bounds__(128, NR > 0 ? 5 : 7) pack_sweep_rec(const __grid_constant__ RecordParams<T> q) {
+    step_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (c * Pack<T>::W >= q.f.room.nz || j >= q.f.room.ny) return;
@@ -49,28 +52,29 @@ __global__ void __launch_bounds__(128, NR > 0 ? 5 : 7) pack_sweep_rec(const __gr
 }
 
 template <bool L, bool W, int NR>
-void launch_one(const FusedParams<double> &f, dim3 grid, dim3 block, cudaStream_t st) {
-    pack_sweep<L, W, NR><<<grid, block, 0, st>>>(f);
+void launch_one(const FusedParams<double> &f, dim3 grid, dim3 block, bool early, cudaStream_t st) {
+    if (early) launch_after(pack_sweep<L, W, NR>, grid, block, st, f);
+    else pack_sweep<L, W, NR><<<grid, block, 0, st>>>(f);
 }
 template <bool L, bool W, int NR, typename T>
-void launch_one(const RecordParams<T> &q, dim3 grid, dim3 block, cudaStream_t st) {
-    pack_sweep_rec<T, L, W, NR><<<grid, block, 0, st>>>(q);
+void launch_one(const RecordParams<T> &q, dim3 grid, dim3 block, bool, cudaStream_t st) {
+    launch_after(pack_sweep_rec<T, L, W, NR>, grid, block, st, q);
 }
 
 template <bool L, bool W, typename P>
-void launch_relax(const P &p, int n_relax, dim3 grid, dim3 block, cudaStream_t st) {
+void launch_relax(const P &p, int n_relax, dim3 grid, dim3 block, bool early, cudaStream_t st) {
     switch (n_relax) {
-        case 0: launch_one<L, W, 0>(p, grid, block, st); break;
-        case 1: launch_one<L, W, 1>(p, grid, block, st); break;
-        case 2: launch_one<L, W, 2>(p, grid, block, st); break;
-        case 3: launch_one<L, W, 3>(p, grid, block, st); break;
-        default: launch_one<L, W, 4>(p, grid, block, st); break;
+        case 0: launch_one<L, W, 0>(p, grid, block, early, st); break;
+        case 1: launch_one<L, W, 1>(p, grid, block, early, st); break;
+        case 2: launch_one<L, W, 2>(p, grid, block, early, st); break;
+        case 3: launch_one<L, W, 3>(p, grid, block, early, st); break;
+        default: launch_one<L, W, 4>(p, grid, block, early, st); break;
     }
 }
 
 template <typename T, typename P>
 void launch_room(const Room<T> &room, int planes, const P &p, bool layer, bool walls, int n_relax,
-                 int block_threads, cudaStream_t st) {
+                 int block_threads, bool early, cudaStream_t st) {
     const int chunks = (room.nz + Pack<T>::W - 1) / Pack<T>::W;
     int bx = 1;
     while (bx < chunks && bx < 32) bx <<= 1;
@@ -78,25 +82,25 @@ void launch_room(const Room<T> &room, int planes, const P &p, bool layer, bool w
     const dim3 block(bx, by, 1);
     const dim3 grid((chunks + bx - 1) / bx, (room.ny + by - 1) / by, (room.nx + planes - 1) / planes);
     if (layer) {
-        if (walls) launch_relax<true, true>(p, n_relax, grid, block, st);
-        else launch_relax<true, false>(p, n_relax, grid, block, st);
+        if (walls) launch_relax<true, true>(p, n_relax, grid, block, early, st);
+        else launch_relax<true, false>(p, n_relax, grid, block, early, st);
     } else {
-        if (walls) launch_relax<false, true>(p, n_relax, grid, block, st);
-        else launch_relax<false, false>(p, n_relax, grid, block, st);
+        if (walls) launch_relax<false, true>(p, n_relax, grid, block, early, st);
+        else launch_relax<false, false>(p, n_relax, grid, block, early, st);
     }
 }
 
 }  // namespace
 
 void launch_pack_sweep(const FusedParams<double> &f, bool layer, bool walls, int n_relax, int block_threads,
-                       cudaStream_t st) {
-    launch_room(f.room, f.planes, f, layer, walls, n_relax, block_threads, st);
+                       bool early, cudaStream_t st) {
+    launch_room(f.room, f.planes, f, layer, walls, n_relax, block_threads, early, st);
 }
 
 template <typename T>
 void launch_pack_rec(const FusedParams<T> &f, const History<T> &history, bool layer, bool walls, int n_relax,
                      int block_threads, cudaStream_t st) {
-    launch_room(f.room, f.planes, RecordParams<T>{f, history}, layer, walls, n_relax, block_threads, st);
+    launch_room(f.room, f.planes, RecordParams<T>{f, history}, layer, walls, n_relax, block_threads, true, st);
 }
 
 template void launch_pack_rec<float>(const FusedParams<float> &, const History<float> &, bool, bool, int, int,

@@ -8,9 +8,10 @@
 namespace acf {
 
 // One fused step of one room (or slab) from f.room's copy to the next, `f.planes` x planes and up
-// to `block_threads` threads per block.
+// to `block_threads` threads per block. `early`: as launch_after does (not in a slab group, whose
+// streams wait on one another's events between the launches).
 void launch_pack_sweep(const FusedParams<double> &f, bool layer, bool walls, int n_relax, int block_threads,
-                       cudaStream_t stream);
+                       bool early, cudaStream_t stream);
 
 // The same step, also writing the forward history of the gradients.
 template <typename T>

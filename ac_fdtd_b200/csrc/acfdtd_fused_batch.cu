@@ -16,6 +16,7 @@
 #include "acfdtd_fused.cuh"
 
 #include "acfdtd_fused_kernel.cuh"
+#include "acfdtd_host.cuh"
 
 namespace acf {
 namespace {
@@ -25,13 +26,13 @@ namespace {
 template <typename T, bool LAYER, bool WALLS, int NR, bool REC>
 __global__ void __launch_bounds__(kPackThreads, pack_batch_blocks(sizeof(T), NR > 0, REC))
 pack_batch(const FusedBatchParams<T> b) {
+    step_next();
     constexpr int kWords = sizeof(FusedParams<T>) / sizeof(int), kHistoryWords = sizeof(History<T>) / sizeof(int);
     static_assert(sizeof(FusedParams<T>) % sizeof(int) == 0 && sizeof(History<T>) % sizeof(int) == 0, "whole words");
     __shared__ __align__(16) int raw[kWords + (REC ? kHistoryWords : 0)];
     const FusedParams<T> &f = *reinterpret_cast<const FusedParams<T> *>(raw);
     static_assert(kWords % 2 == 0, "the history is 8-byte aligned");
     const History<T> *history = REC ? reinterpret_cast<const History<T> *>(raw + kWords) : nullptr;
-    const int64_t step = *b.step_base + b.local_step;
     int staged = -1;
     for (int t = blockIdx.x; t < b.n_tiles; t += gridDim.x) {
         const Tile tile = b.tiles[t];
@@ -46,6 +47,8 @@ pack_batch(const FusedBatchParams<T> b) {
             __syncthreads();
             staged = tile.room;
         }
+        step_wait();                             // tiles and descriptions are only written by the host
+        const int64_t step = *b.step_base + b.local_step;
         if ((int)threadIdx.x < tile.count) {
             const int pack = tile.first + threadIdx.x, packs = (f.room.nz + Pack<T>::W - 1) / Pack<T>::W;
             pack_column<T, LAYER, WALLS, NR, REC>(f, tile.i_begin, tile.i_end, pack / packs, pack % packs, step,
@@ -57,11 +60,11 @@ pack_batch(const FusedBatchParams<T> b) {
 template <typename T, bool L, bool W, bool R>
 void launch_relax(const FusedBatchParams<T> &p, int n_relax, dim3 grid, dim3 block, cudaStream_t st) {
     switch (n_relax) {
-        case 0: pack_batch<T, L, W, 0, R><<<grid, block, 0, st>>>(p); break;
-        case 1: pack_batch<T, L, W, 1, R><<<grid, block, 0, st>>>(p); break;
-        case 2: pack_batch<T, L, W, 2, R><<<grid, block, 0, st>>>(p); break;
-        case 3: pack_batch<T, L, W, 3, R><<<grid, block, 0, st>>>(p); break;
-        default: pack_batch<T, L, W, 4, R><<<grid, block, 0, st>>>(p); break;
+        case 0: launch_after(pack_batch<T, L, W, 0, R>, grid, block, st, p); break;
+        case 1: launch_after(pack_batch<T, L, W, 1, R>, grid, block, st, p); break;
+        case 2: launch_after(pack_batch<T, L, W, 2, R>, grid, block, st, p); break;
+        case 3: launch_after(pack_batch<T, L, W, 3, R>, grid, block, st, p); break;
+        default: launch_after(pack_batch<T, L, W, 4, R>, grid, block, st, p); break;
     }
 }
 
