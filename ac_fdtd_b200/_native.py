@@ -45,7 +45,7 @@ EXPORTED_SYMBOLS = (
     "acf_solver_device", "acf_energy_terms_planes", "acf_run_slabs", "acf_batch_device_status",
     "acf_set_wait_test", "acf_schroeder_decay", "acf_decay_fit", "acf_clarity",
     "acf_spectral_divide", "acf_pressure_only_energy_terms", "acf_set_time_blocking",
-    "acf_get_time_blocking",
+    "acf_get_time_blocking", "acf_adjoint_wall_gradients", "acf_batch_adjoint_wall_gradients",
 )
 
 SCHEME_TWO_SWEEPS, SCHEME_FUSED, SCHEME_FUSED_STAGED, SCHEME_PRESSURE_ONLY = 0, 1, 2, 3
@@ -151,6 +151,9 @@ _SIGNATURES = {
     "acf_clarity": (ctypes.c_int, [_P, _I64, _I64, _I64, _P, _P]),
     "acf_spectral_divide": (ctypes.c_int, [_P, _P, _I64, _I64, ctypes.c_double, ctypes.c_double,
                                            ctypes.c_double, _P, _P, _P]),
+    "acf_adjoint_wall_gradients": (ctypes.c_int, [_P, ctypes.c_double, ctypes.c_int32, _DP, _DP, _P]),
+    "acf_batch_adjoint_wall_gradients": (ctypes.c_int, [_P, ctypes.c_int32, ctypes.c_double,
+                                                        ctypes.c_int32, _DP, _DP, _P]),
     "acf_batch_adjoint_prepare": (ctypes.c_int, [_P, _I64]),
     "acf_batch_adjoint_shell_size": (ctypes.c_int64, [_P, ctypes.c_int32]),
     "acf_batch_forward_record": (ctypes.c_int, [_P, _I64, _I64, _P]),

@@ -105,6 +105,18 @@ def wall_gradients(walls, shape, grad_a, sound_speed, dt, dx):
     return np.array([m.sum() for m in cells]), cells
 
 
+def _wall_gradients_of_run(call, walls, shape, sound_speed, dt, dx):
+    """``wall_gradients`` of the run ``call(scale, patches, cells, sums)`` belongs to, mapped and
+    summed on the device."""
+    patches = int(walls.patches) if hasattr(walls, "patch_values") else 1
+    faces = [tuple(n for a, n in enumerate(shape) if a != axis) for axis, _ in FACES]
+    ends = np.cumsum([b * c for b, c in faces])
+    flat, sums = np.empty(int(ends[-1])), np.empty((6, patches, patches))
+    call(sound_speed * dt / (2.0 * dx), patches, _as_double_pointer(flat), _as_double_pointer(sums))
+    cells = [m.reshape(face) for m, face in zip(np.split(flat, ends[:-1]), faces)]
+    return (sums if hasattr(walls, "patch_values") else sums.reshape(6)), cells
+
+
 def _air_chain(processes, c, rho, dx, dt, dgain, dmean, ddecay, dscale):
     """dL/dDelta_r and dL/dtau_r from the gradients of the scheme's relaxation coefficients.
 
@@ -152,7 +164,6 @@ class DifferentiableRoom:
         _native.check(lib.acf_adjoint_prepare(self.solver._handle, flags, self.max_steps,
                                               int(checkpoint_every or 0)), "acf_adjoint_prepare")
         self.checkpoint_every = int(lib.acf_adjoint_checkpoint_interval(self.solver._handle))
-        self._shell_size = int(lib.acf_adjoint_shell_size(self.solver._handle))
         self.n_steps = 0
 
     @property
@@ -188,21 +199,22 @@ class DifferentiableRoom:
         grad = np.ascontiguousarray(grad_recordings, dtype=np.float64).reshape(len(s._receivers), n)
         n_src = len(s._sources)
         grad_src = np.zeros((n_src, n))
-        grad_shell = np.zeros(self._shell_size) if "walls" in self.wrt else None
         n_air = 3 * s.n_relax + 1
         grad_air = np.zeros(n_air) if "air" in self.wrt else None
 
         def ptr(a):
             return None if a is None else _as_double_pointer(a)
 
-        _native.check(s._lib.acf_adjoint_run(s._handle, ptr(grad), ptr(grad_src), ptr(grad_shell),
+        _native.check(s._lib.acf_adjoint_run(s._handle, ptr(grad), ptr(grad_src), None,
                                              ptr(grad_air), s._stream), "acf_adjoint_run")
         out = RoomGradients(signal=grad_src)
         block = s.coefficients
         c, rho = float(s.medium.sound_speed), float(s.medium.density)
-        if grad_shell is not None:
-            out.walls, out.wall_cells = wall_gradients(s.walls, block.shape, grad_shell, c,
-                                                       block.dt, block.dx)
+        if "walls" in self.wrt:
+            out.walls, out.wall_cells = _wall_gradients_of_run(
+                lambda *args: _native.check(s._lib.acf_adjoint_wall_gradients(s._handle, *args, s._stream),
+                                            "acf_adjoint_wall_gradients"),
+                s.walls, block.shape, c, block.dt, block.dx)
         if grad_air is not None:
             R = s.n_relax
             dgain, dmean, ddecay, dscale = grad_air[:R], grad_air[R:2 * R], grad_air[2 * R:3 * R], grad_air[3 * R]
@@ -229,8 +241,6 @@ class DifferentiableBatch:
         lib = self.batch._lib
         _native.check(lib.acf_batch_adjoint_prepare(self.batch._handle, self.max_steps),
                       "acf_batch_adjoint_prepare")
-        self._shell_sizes = [int(lib.acf_batch_adjoint_shell_size(self.batch._handle, r))
-                             for r in range(len(self.batch))]
         self.n_steps = 0
 
     def set_walls(self, room: int, walls) -> None:
@@ -261,24 +271,21 @@ class DifferentiableBatch:
              for r, g in enumerate(grad_recordings)], axis=0))
         n_src = sum(len(s) for s in b._sources)
         grad_src = np.zeros((max(n_src, 1), n))
-        grad_shell = np.zeros(sum(self._shell_sizes))
         _native.check(b._lib.acf_batch_adjoint_run(b._handle, _as_double_pointer(grad),
-                                                   _as_double_pointer(grad_src),
-                                                   _as_double_pointer(grad_shell), b._stream),
+                                                   _as_double_pointer(grad_src), None, b._stream),
                       "acf_batch_adjoint_run")
         out = []
-        src_row = shell_at = 0
+        src_row = 0
         for r in range(len(b)):
             block, spec = b.blocks[r], b.specs[r]
             medium = spec.get("medium", AIR)
             k = len(b._sources[r])
             g = RoomGradients(signal=grad_src[src_row:src_row + k])
             src_row += k
-            shell = grad_shell[shell_at:shell_at + self._shell_sizes[r]]
-            shell_at += self._shell_sizes[r]
-            g.walls, g.wall_cells = wall_gradients(spec.get("walls") or WallAdmittances(),
-                                                   block.shape, shell,
-                                                   float(medium.sound_speed), block.dt, block.dx)
+            g.walls, g.wall_cells = _wall_gradients_of_run(
+                lambda *args: _native.check(b._lib.acf_batch_adjoint_wall_gradients(b._handle, r, *args, b._stream),
+                                            "acf_batch_adjoint_wall_gradients"),
+                spec.get("walls") or WallAdmittances(), block.shape, float(medium.sound_speed), block.dt, block.dx)
             out.append(g)
         return out
 

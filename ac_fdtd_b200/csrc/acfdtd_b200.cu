@@ -55,6 +55,7 @@
 #include "acfdtd_device.cuh"
 #include "acfdtd_host.cuh"
 #include "acfdtd_fused.cuh"
+#include "acfdtd_shell.cuh"
 #include "acfdtd_resident.cuh"
 
 using namespace acf;
@@ -3470,8 +3471,8 @@ struct acf_batch {
         int32_t every = 0;           // checkpoint interval
         int64_t recorded = 0, step0 = 0;
         bool fields_recorded = false;   // the recorded run wrote D and psi of every step itself
-        int direct_mode = -1;        // how the last recorded run stepped (graph validity): 0 two
-                                     // sweeps, 1 two sweeps writing D and psi, 2 the lean step
+        int direct_mode = -1;        // how the last recorded run stepped (graph validity): 1 for
+                                     // writing D and psi, plus 2 for one sweep per step
         int64_t shell_total = 0;
         int64_t face_off[6] = {};
         void *hist_shell = nullptr;  // capacity x 2 x shell_total values
@@ -3496,6 +3497,8 @@ struct acf_batch {
     };
     std::vector<RoomAdjoint> badj;
     int64_t badj_capacity = 0, badj_recorded = 0, badj_step0 = 0;
+    double *wall_scratch = nullptr;  // wall_gradients: the faces' maps and sums
+    int64_t wall_scratch_size = 0;
     void *badj_history = nullptr;    // device array of History<T>, one per room
     void *badj_table = nullptr;      // device array of AdjointParams<T>: 2 per room (the two copies of mu)
 
@@ -4472,6 +4475,7 @@ void free_batch(acf_batch *b) {
     }
     dev_free(b->badj_table);
     dev_free(b->badj_history);
+    dev_free(b->wall_scratch);
     dev_free(b->pair_ring);
     dev_free(b->pair_progress);
     dev_free(b->psi2);
@@ -6152,6 +6156,31 @@ int batch_adjoint_impl(acf_batch *b, const double *grad_rec, double *grad_src, d
     return ACF_OK;
 }
 
+// The maps of the six faces and their sums per patch from the last adjoint run's boundary sums.
+int wall_gradients(acf_batch *b, const RoomHost &h, const double *grad_shell, int64_t shell_total, double scale,
+                   int32_t patches, double *cells, double *sums, cudaStream_t st) {
+    if (!cells || !sums) return fail(ACF_ERR_ARGUMENT, "null output");
+    if (patches < 1 || patches > 1024) return fail(ACF_ERR_ARGUMENT, "patches must be in [1, 1024], got %d", patches);
+    const int64_t n_sums = (int64_t)6 * patches * patches, need = shell_total + n_sums;
+    if (need > b->wall_scratch_size) {
+        ACF_CUDA(cudaStreamSynchronize(st));
+        dev_free(b->wall_scratch);
+        b->wall_scratch = nullptr;
+        b->wall_scratch_size = 0;
+        ACF_CUDA(dev_malloc(&b->wall_scratch, (size_t)need * sizeof(double)));
+        b->wall_scratch_size = need;
+    }
+    const int32_t n[3] = {(int32_t)h.nx, (int32_t)h.ny, (int32_t)h.nz};
+    int rc = shell_gradients(grad_shell, n, scale, patches, b->wall_scratch, b->wall_scratch + shell_total, st);
+    if (rc) return rc;
+    b->launches += 2;
+    ACF_CUDA(cudaMemcpyAsync(cells, b->wall_scratch, (size_t)shell_total * sizeof(double), cudaMemcpyDeviceToHost, st));
+    ACF_CUDA(cudaMemcpyAsync(sums, b->wall_scratch + shell_total, (size_t)n_sums * sizeof(double),
+                             cudaMemcpyDeviceToHost, st));
+    ACF_CUDA(cudaStreamSynchronize(st));
+    return ACF_OK;
+}
+
 }  // namespace
 
 // ==========================================================================================
@@ -6471,6 +6500,17 @@ int acf_adjoint_run(acf_solver *h, const double *grad_rec, double *grad_src, dou
                              : adjoint_impl<float>(h, grad_rec, grad_src, grad_shell, grad_air, st);
 }
 
+int acf_adjoint_wall_gradients(acf_solver *h, double scale, int32_t patches, double *cells, double *sums,
+                               acf_stream stream) {
+    if (!h) return fail(ACF_ERR_ARGUMENT, "null solver");
+    if (!h->adj.fields || h->adj.recorded < 1) return fail(ACF_ERR_STATE, "no recorded forward run");
+    if (!h->adj.grad_shell)
+        return fail(ACF_ERR_STATE, "wall gradients need a room with wall coefficients and ACF_GRAD_WALLS");
+    DeviceGuard guard(h->device);
+    return wall_gradients(h, h->rooms[0], h->adj.grad_shell, h->adj.shell_total, scale, patches, cells, sums,
+                          (cudaStream_t)stream);
+}
+
 int acf_adjoint_download(acf_solver *h, int field, void *dst, acf_stream stream) {
     if (!h || !dst) return fail(ACF_ERR_ARGUMENT, "null argument");
     if (!h->adj.fields) return fail(ACF_ERR_STATE, "call acf_adjoint_prepare first");
@@ -6628,6 +6668,17 @@ int acf_batch_adjoint_run(acf_batch *b, const double *grad_rec, double *grad_src
     cudaStream_t st = (cudaStream_t)stream;
     return b->precision == 8 ? batch_adjoint_impl<double>(b, grad_rec, grad_src, grad_shell, st)
                              : batch_adjoint_impl<float>(b, grad_rec, grad_src, grad_shell, st);
+}
+
+int acf_batch_adjoint_wall_gradients(acf_batch *b, int32_t room, double scale, int32_t patches, double *cells,
+                                     double *sums, acf_stream stream) {
+    int rc = check_room(b, room);
+    if (rc) return rc;
+    if (b->badj.empty() || b->badj_recorded < 1) return fail(ACF_ERR_STATE, "no recorded forward run");
+    DeviceGuard guard(b->device);
+    const auto &ra = b->badj[(size_t)room];
+    return wall_gradients(b, b->rooms[(size_t)room], ra.grad_shell, ra.shell_total, scale, patches, cells, sums,
+                          (cudaStream_t)stream);
 }
 
 int acf_batch_reset_state(acf_batch *b, acf_stream stream) {

@@ -259,17 +259,23 @@ int acf_energy_terms_planes(acf_solver *solver, double dx, int64_t x_begin, int6
  * -- the recorded run then keeps them and nothing is recomputed -- else ceil(sqrt(max_steps)).
  *
  * acf_adjoint_prepare  allocates the history for runs of up to max_steps steps.
- * acf_forward_record   is acf_run that also writes that history (and the checkpoints). In
- *                      single precision with nz a multiple of 4 and no air gradients it takes one
- *                      lean sweep per step into the second copy of p and v -- allocated on the
- *                      first such call when the scheme has none -- and leaves the state in the
- *                      primary copy; results equal the two-sweep record bit for bit.
+ * acf_forward_record   is acf_run that also writes that history (and the checkpoints). Unless it
+ *                      writes checkpoints it takes one fused sweep per step into the second copy
+ *                      of p and v -- allocated on the first such call when the scheme has none;
+ *                      two sweeps in place where the device has no memory for it -- and leaves
+ *                      the state in the primary copy; results equal the two-sweep record bit for
+ *                      bit.
  * acf_adjoint_run      takes dL/drec (n_receivers rows of n_steps doubles, host) and returns
  *                      (each optional, host, FP64): dL/dsignal (n_sources rows of n_steps),
  *                      dL/da per boundary cell (acf_adjoint_shell_size entries, shell order of
  *                      the wall coefficients with each cell on the first face it touches), and
  *                      the air sums (dL/dgain_r, dL/dmean_r, dL/ddecay_r for r < n_relax, then
  *                      dL/drelax_scale).
+ * acf_adjoint_wall_gradients returns, of the last acf_adjoint_run and on its stream, the wall maps:
+ *                      scale dL/da at every cell of each face in turn (acf_adjoint_shell_size
+ *                      doubles; a cell on an edge counts on each of its faces), and their sums
+ *                      over the patches x patches patches of each face (6 patches^2 doubles; 1
+ *                      for whole walls). Host memory, FP64.
  * acf_adjoint_download returns dL/d of the initial state, field by field.
  * acf_set_coefficients swaps in new coefficients (same grid, precision, relaxation count and
  *                      the same presence of layer and walls) without touching the state. */
@@ -286,6 +292,8 @@ int acf_forward_record(acf_solver *solver, int64_t n_steps, int64_t step_offset,
                        acf_stream stream);
 int acf_adjoint_run(acf_solver *solver, const double *grad_rec, double *grad_src,
                     double *grad_shell, double *grad_air, acf_stream stream);
+int acf_adjoint_wall_gradients(acf_solver *solver, double scale, int32_t patches, double *cells,
+                               double *sums, acf_stream stream);
 int acf_adjoint_download(acf_solver *solver, int field, void *dst, acf_stream stream);
 
 /* Energy sums without any allocation. No counterpart in the reference.
@@ -440,6 +448,8 @@ int acf_batch_forward_record(acf_batch *batch, int64_t n_steps, int64_t step_off
                              acf_stream stream);
 int acf_batch_adjoint_run(acf_batch *batch, const double *grad_rec, double *grad_src,
                           double *grad_shell, acf_stream stream);
+int acf_batch_adjoint_wall_gradients(acf_batch *batch, int32_t room, double scale, int32_t patches,
+                                     double *cells, double *sums, acf_stream stream);
 int acf_batch_reset_state(acf_batch *batch, acf_stream stream);
 int acf_batch_set_coefficients(acf_batch *batch, int32_t room, const acf_config *config);
 
