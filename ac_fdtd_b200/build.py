@@ -20,11 +20,12 @@ PACKAGE = Path(__file__).resolve().parent
 ROOT = PACKAGE.parent
 CSRC = PACKAGE / "csrc"
 _SHARED = [CSRC / "acfdtd_device.cuh", CSRC / "acfdtd_host.cuh", CSRC / "acfdtd_resident.cuh",
-           CSRC / "acfdtd_fused.cuh", CSRC / "acfdtd_shell.cuh", ROOT / "include" / "acfdtd_b200.h"]
+           CSRC / "acfdtd_fused.cuh", CSRC / "acfdtd_adjoint.cuh", CSRC / "acfdtd_shell.cuh", ROOT / "include" / "acfdtd_b200.h"]
 #: Every source with the headers it includes.
 SOURCES = {CSRC / "acfdtd_b200.cu": _SHARED,
            CSRC / "acfdtd_fused.cu": [*_SHARED, CSRC / "acfdtd_pack.cuh", CSRC / "acfdtd_fused_kernel.cuh"],
            CSRC / "acfdtd_fused_batch.cu": [*_SHARED, CSRC / "acfdtd_pack.cuh", CSRC / "acfdtd_fused_kernel.cuh"],
+           CSRC / "acfdtd_adjoint.cu": [*_SHARED, CSRC / "acfdtd_pack.cuh"],
            CSRC / "acfdtd_shell.cu": [CSRC / "acfdtd_shell.cuh", CSRC / "acfdtd_host.cuh",
                                       ROOT / "include" / "acfdtd_b200.h"],
            CSRC / "acfdtd_post.cu": [CSRC / "acfdtd_host.cuh", ROOT / "include" / "acfdtd_b200.h"]}

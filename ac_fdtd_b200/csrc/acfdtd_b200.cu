@@ -54,6 +54,7 @@
 #include "acfdtd_b200.h"
 #include "acfdtd_device.cuh"
 #include "acfdtd_host.cuh"
+#include "acfdtd_adjoint.cuh"
 #include "acfdtd_fused.cuh"
 #include "acfdtd_shell.cuh"
 #include "acfdtd_resident.cuh"
@@ -2063,44 +2064,13 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 8 ? 2 : 3)) pressure_batch(
 // where u = 1/(1+a), q = a/(1+a), h and g the layer products, S = dt sum G. The gradient of the
 // wall closed form p_hat = u p_tilde - q p with respect to a is -u^2 (p_tilde + p).
 
-template <typename T>
-struct AdjointParams {
-    Room<T> room;                  // coefficients, geometry, profiles, walls, points
-    T *lp, *lvx, *lvy, *lvz, *lpsi, *ld;  // adjoint fields (room geometry)
-    const double *grad_rec;        // n_rec rows of grad_stride, column = step - grad_step0
-    double *grad_src;              // n_src rows of grad_stride
-    int64_t grad_stride, grad_step0;
-    History<T> hist;
-    double *grad_shell;            // FP64 dL/da per boundary cell (shell index)
-    double *air_partials;          // per block: G_r (R), m_r (R), delta_r (R), S
-    const int64_t *step_base;      // the forward step reversed is *step_base + local_step
-    int32_t local_step;
-    int32_t planes;
-    int32_t air;                   // accumulate air gradients (needs hist.fields)
-    // Fused adjoint step only: mu^{n+1} and lambda_D^n go to these (the other copies); lvx..lvz
-    // hold mu^{n+2} and ld holds lambda_D^{n+1}.
-    T *out_vx, *out_vy, *out_vz, *out_d;
-};
-
-// mu on a face: (LV + (lambda_D[lower cell] - lambda_D[upper cell])) g_a g_b g_c, the face
-// sweep's arithmetic, with lambda_D = 0 outside the room (x - 0 == x exactly, so the far faces'
-// LV + lambda_D[lower] is reproduced bit for bit).
-template <typename T, bool LAYER>
-__device__ __forceinline__ T adjoint_face(T lv, T d_lower, T d_upper, T ga, T gb, T gc) {
-    T m = lv + (d_lower - d_upper);
-    if (LAYER) m = ((m * ga) * gb) * gc;
-    return m;
-}
-
 // One (row j, chunk c) column of the adjoint pressure sweep over planes [i_begin, i_end),
 // reversing forward step `step`; air-gradient terms are added to `air_acc`.
 //
-// FUSED also performs the face sweep of the step after (forward step + 1) first: mu^{n+1} on the
-// cell's six faces from mu^{n+2} (lvx..lvz) and lambda_D^{n+1} (ld) -- its own three lower faces
-// (stored, with the far boundary faces) and its three upper faces (recomputed exactly as their
-// owners compute them) -- and writes lambda_D^n to out_d. Per cell and step this moves (10 + 2R)
-// elements instead of the two sweeps' (13 + 2R), with the same results.
-template <typename T, bool LAYER, bool WALLS, int NR, bool AIR, bool FUSED = false, int VW = kVec>
+// It is the last recorded step's; the steps before it, whose face sweep comes first, are one fused
+// launch each (acfdtd_adjoint.cu, and lean_adjoint_column), which moves (10 + 2R) elements per cell
+// instead of the two sweeps' (13 + 2R).
+template <typename T, bool LAYER, bool WALLS, int NR, bool AIR, int VW = kVec>
 __device__ __forceinline__ void adjoint_pressure_column(const AdjointParams<T> &a, int i_begin,
                                                         int i_end, int j, int c, int64_t step,
                                                         T *air_acc) {
@@ -2114,36 +2084,11 @@ __device__ __forceinline__ void adjoint_pressure_column(const AdjointParams<T> &
     const bool any_mine = points != 0 || all_points;
     const bool wall_column = j == 0 || j == s.ny - 1 || k0 == 0 || k0 + VW >= s.nz;
     T XL[VW];
-    // FUSED: lambda_D^{n+1} of the current cell and of the cell below in x, carried along x
-    T Dc[VW], Dm[VW];
-    T fj_cell = T(1), fj_face = T(1), fj1_face = T(1);
-    if (FUSED) {
-        const int64_t b0 = (int64_t)i_begin * s.plane + column;
-        VecW<T, VW>::ldg(a.ld + b0, Dc);
-#pragma unroll
-        for (int e = 0; e < VW; e++) Dm[e] = T(0);
-        if (i_begin > 0) VecW<T, VW>::ldg(a.ld + b0 - s.plane, Dm);
-        if (LAYER) {
-            fj_cell = __ldg(s.cell[1] + j);
-            fj_face = __ldg(s.face[1] + j);
-            fj1_face = __ldg(s.face[1] + j + 1);
-        }
-        T V[VW];
-        VecW<T, VW>::ldg(a.lvx + b0, V);
-        const T fi_face = LAYER ? __ldg(s.face[0] + i_begin) : T(1);
-#pragma unroll
-        for (int e = 0; e < VW; e++)
-            XL[e] = k0 + e < s.nz ? adjoint_face<T, LAYER>(V[e], Dm[e], Dc[e], fi_face, fj_cell,
-                                                           LAYER ? __ldg(s.cell[2] + k0 + e) : T(1))
-                                  : V[e];
-    } else {
-        VecW<T, VW>::ldg(a.lvx + (int64_t)i_begin * s.plane + column, XL);
-    }
+    VecW<T, VW>::ldg(a.lvx + (int64_t)i_begin * s.plane + column, XL);
     for (int i = i_begin; i < i_end; i++) {
         const int64_t base = (int64_t)i * s.plane + column;
         if (s.prefetch && i + 1 < i_end) {  // the next plane's own-row inputs into L2
             const int64_t next = base + s.plane;
-            if (FUSED && i + 2 < s.nx) prefetch_l2(a.ld + next + s.plane);
             prefetch_l2(a.lvx + next + s.plane);
             prefetch_l2(a.lvy + next);
             prefetch_l2(a.lvz + next);
@@ -2159,64 +2104,11 @@ __device__ __forceinline__ void adjoint_pressure_column(const AdjointParams<T> &
         }
         T XH[VW], YL[VW], YH[VW], Z[VW], L[VW], LS[NR > 0 ? NR : 1][VW];
         T above;
-        T Dxp[VW];   // FUSED: lambda_D^{n+1} of the next plane
-        if (FUSED) {
-            T Dy[VW], Dyp[VW], VXp[VW], VY[VW], VYp[VW], VZ[VW];
-#pragma unroll
-            for (int e = 0; e < VW; e++) {
-                Dxp[e] = T(0);
-                Dy[e] = T(0);
-                Dyp[e] = T(0);
-            }
-            if (i + 1 < s.nx) VecW<T, VW>::ldg(a.ld + base + s.plane, Dxp);
-            if (j > 0) VecW<T, VW>::ldg(a.ld + base - s.pz, Dy);
-            if (j + 1 < s.ny) VecW<T, VW>::ldg(a.ld + base + s.pz, Dyp);
-            const T d_below = k0 > 0 ? __ldg(a.ld + base - 1) : T(0);
-            const T d_above = k0 + VW < s.nz ? __ldg(a.ld + base + VW) : T(0);
-            VecW<T, VW>::ldg(a.lvx + base + s.plane, VXp);
-            VecW<T, VW>::ldg(a.lvy + base, VY);
-            VecW<T, VW>::ldg(a.lvy + base + s.pz, VYp);
-            VecW<T, VW>::ldg(a.lvz + base, VZ);
-            const T vz_above = has_above ? __ldg(a.lvz + base + VW) : T(0);
-            T fi_cell = T(1), fi1_face = T(1);
-            if (LAYER) {
-                fi_cell = __ldg(s.cell[0] + i);
-                fi1_face = __ldg(s.face[0] + i + 1);
-            }
-#pragma unroll
-            for (int e = 0; e < VW; e++) {
-                const int k = k0 + e;
-                const T gk_cell = LAYER ? __ldg(s.cell[2] + min(k, s.nz - 1)) : T(1);
-                if (k < s.nz) {
-                    XH[e] = adjoint_face<T, LAYER>(VXp[e], Dc[e], Dxp[e], fi1_face, fj_cell, gk_cell);
-                    YL[e] = adjoint_face<T, LAYER>(VY[e], Dy[e], Dc[e], fi_cell, fj_face, gk_cell);
-                    YH[e] = adjoint_face<T, LAYER>(VYp[e], Dc[e], Dyp[e], fi_cell, fj1_face, gk_cell);
-                } else {
-                    XH[e] = VXp[e];
-                    YL[e] = VY[e];
-                    YH[e] = VYp[e];
-                }
-                // z face k: between cells k - 1 and k; the top face k = nz has only the lower one
-                if (k <= s.nz) {
-                    const T lower = k > 0 ? (e == 0 ? d_below : Dc[e - 1]) : T(0);
-                    const T upper = k < s.nz ? Dc[e] : T(0);
-                    Z[e] = adjoint_face<T, LAYER>(VZ[e], lower, upper, fi_cell, fj_cell,
-                                                  LAYER ? __ldg(s.face[2] + k) : T(1));
-                } else {
-                    Z[e] = VZ[e];
-                }
-            }
-            above = T(0);
-            if (has_above)
-                above = adjoint_face<T, LAYER>(vz_above, Dc[VW - 1], d_above, fi_cell, fj_cell,
-                                               LAYER ? __ldg(s.face[2] + k0 + VW) : T(1));
-        } else {
-            VecW<T, VW>::ldg(a.lvx + base + s.plane, XH);
-            VecW<T, VW>::ldg(a.lvy + base, YL);
-            VecW<T, VW>::ldg(a.lvy + base + s.pz, YH);
-            VecW<T, VW>::ldg(a.lvz + base, Z);
-            above = has_above ? __ldg(a.lvz + base + VW) : T(0);
-        }
+        VecW<T, VW>::ldg(a.lvx + base + s.plane, XH);
+        VecW<T, VW>::ldg(a.lvy + base, YL);
+        VecW<T, VW>::ldg(a.lvy + base + s.pz, YH);
+        VecW<T, VW>::ldg(a.lvz + base, Z);
+        above = has_above ? __ldg(a.lvz + base + VW) : T(0);
         VecW<T, VW>::load(a.lp + base, L);
 #pragma unroll
         for (int r = 0; r < NR; r++) VecW<T, VW>::load(a.lpsi + r * s.field + base, LS[r]);
@@ -2329,22 +2221,7 @@ __device__ __forceinline__ void adjoint_pressure_column(const AdjointParams<T> &
         VecW<T, VW>::store(a.lp + base, L);
 #pragma unroll
         for (int r = 0; r < NR; r++) VecW<T, VW>::store(a.lpsi + r * s.field + base, LS[r]);
-        if (FUSED) {
-            VecW<T, VW>::store(a.out_d + base, LD);
-            VecW<T, VW>::store(a.out_vx + base, XL);
-            VecW<T, VW>::store(a.out_vy + base, YL);
-            VecW<T, VW>::store(a.out_vz + base, Z);
-            if (i == s.nx - 1) VecW<T, VW>::store(a.out_vx + base + s.plane, XH);
-            if (j == s.ny - 1) VecW<T, VW>::store(a.out_vy + base + s.pz, YH);
-            if (k0 + VW == s.nz) a.out_vz[base + VW] = above;
-#pragma unroll
-            for (int e = 0; e < VW; e++) {
-                Dm[e] = Dc[e];
-                Dc[e] = Dxp[e];
-            }
-        } else {
-            VecW<T, VW>::store(a.ld + base, LD);
-        }
+        VecW<T, VW>::store(a.ld + base, LD);
 #pragma unroll
         for (int e = 0; e < VW; e++) XL[e] = XH[e];
     }
@@ -2365,46 +2242,8 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 8 ? (AIR && VW == kVec ? 1 
     for (int t = 0; t < NA; t++) air_acc[t] = T(0);
     if (c < (a.room.nz + VW - 1) / VW && j < a.room.ny) {
         const int i_begin = blockIdx.z * a.planes;
-        adjoint_pressure_column<T, LAYER, WALLS, NR, AIR, false, VW>(a, i_begin, min(a.room.nx, i_begin + a.planes),
+        adjoint_pressure_column<T, LAYER, WALLS, NR, AIR, VW>(a, i_begin, min(a.room.nx, i_begin + a.planes),
                                                                      j, c, *a.step_base + a.local_step, air_acc);
-    }
-    if (AIR && NR > 0) {  // uniform per launch: every thread reaches the barrier
-        __shared__ double red[NA][8];
-        const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-        const int lane = tid & 31, warp = tid >> 5;
-        const int n_warps = (blockDim.x * blockDim.y + 31) >> 5;
-#pragma unroll
-        for (int t = 0; t < NA; t++) {
-            double v = (double)air_acc[t];
-            for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
-            if (lane == 0) red[t][warp] = v;
-        }
-        __syncthreads();
-        if (tid < NA) {
-            double v = 0.0;
-            for (int w = 0; w < n_warps; w++) v += red[tid][w];
-            const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-            a.air_partials[block * NA + tid] += v;
-        }
-    }
-}
-
-// The face sweep of forward step n + 1 and the cell sweep of step n in one launch (FUSED above).
-template <typename T, bool LAYER, bool WALLS, int NR, bool AIR, int VW = kVec>
-__global__ void __launch_bounds__(256, (sizeof(T) == 8 ? (AIR && VW == kVec ? 1 : 2) : (AIR && VW == kVec ? 2 : 3)))
-    adjoint_fused_sweep(const AdjointParams<T> a) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    constexpr int NA = 3 * NR + 1;
-    // Per-thread sums over this launch's few cells in the working precision; the block sums
-    // and the sums across blocks and steps are FP64.
-    T air_acc[NA];
-#pragma unroll
-    for (int t = 0; t < NA; t++) air_acc[t] = T(0);
-    if (c < (a.room.nz + VW - 1) / VW && j < a.room.ny) {
-        const int i_begin = blockIdx.z * a.planes;
-        adjoint_pressure_column<T, LAYER, WALLS, NR, AIR, true, VW>(a, i_begin, min(a.room.nx, i_begin + a.planes),
-                                                                    j, c, *a.step_base + a.local_step, air_acc);
     }
     if (AIR && NR > 0) {  // uniform per launch: every thread reaches the barrier
         __shared__ double red[NA][8];
@@ -2857,15 +2696,6 @@ __global__ void __launch_bounds__(256) adjoint_velocity_sweep(const AdjointParam
 // forward batch kernels. Walls and sources only (no air terms).
 
 template <typename T>
-struct BatchAdjointParams {
-    const AdjointParams<T> *rooms;
-    const Tile *tiles;
-    int32_t n_tiles;
-    int32_t local_step;
-    const int64_t *step_base;
-};
-
-template <typename T>
 __device__ __forceinline__ void stage_adjoint(const AdjointParams<T> *src, AdjointParams<T> *dst) {
     static_assert(sizeof(AdjointParams<T>) % sizeof(int) == 0, "whole words");
     const int *from = reinterpret_cast<const int *>(src);
@@ -2917,32 +2747,6 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 8 ? 2 : 3)) adjoint_pressur
             adjoint_pressure_column<T, LAYER, WALLS, NR, false>(*room, tile.i_begin, tile.i_end,
                                                                 pair / room->room.nchunks,
                                                                 pair % room->room.nchunks, step, unused);
-        }
-    }
-}
-
-// The fused adjoint step (face sweep of forward step n + 1, cell sweep of step n) over a batch:
-// each room's parameters name the copy of mu and lambda_D it reads and the one it writes.
-template <typename T, bool LAYER, bool WALLS, int NR>
-__global__ void __maxnreg__(sizeof(T) == 8 ? 168 : 96) adjoint_fused_batch(const BatchAdjointParams<T> b) {
-    __shared__ __align__(16) unsigned char raw[sizeof(AdjointParams<T>)];
-    AdjointParams<T> *room = reinterpret_cast<AdjointParams<T> *>(raw);
-    const int64_t step = *b.step_base + b.local_step;
-    T unused[1];
-    int staged = -1;
-    for (int t = blockIdx.x; t < b.n_tiles; t += gridDim.x) {
-        const Tile tile = b.tiles[t];
-        if (tile.room != staged) {
-            __syncthreads();
-            stage_adjoint(b.rooms + tile.room, room);
-            __syncthreads();
-            staged = tile.room;
-        }
-        if ((int)threadIdx.x < tile.count) {
-            const int pair = tile.first + threadIdx.x;
-            adjoint_pressure_column<T, LAYER, WALLS, NR, false, true>(*room, tile.i_begin, tile.i_end,
-                                                                      pair / room->room.nchunks,
-                                                                      pair % room->room.nchunks, step, unused);
         }
     }
 }
@@ -5351,13 +5155,6 @@ struct AdjPressureAir {
 };
 
 template <typename T, bool L, bool W, int NR>
-struct AdjFused {
-    static void launch(const AdjointParams<T> &p, dim3 g, dim3 b, cudaStream_t st) {
-        adjoint_fused_sweep<T, L, W, NR, false><<<g, b, 0, st>>>(p);
-    }
-};
-
-template <typename T, bool L, bool W, int NR>
 struct LeanAdjFused {
     static void launch(const LeanAdjointParams &p, dim3 g, dim3 b, cudaStream_t st) {
         lean_adjoint_sweep<L, W, NR><<<g, b, 0, st>>>(p);
@@ -5386,14 +5183,6 @@ void fill_adjoint_pairs(float2 *k, const RoomHost &h) {
         put(kAdjDecay + r, (float)h.decay[r]);
     }
 }
-
-template <typename T, bool L, bool W, int NR>
-struct AdjFusedAir {
-    static void launch(const AdjointParams<T> &p, dim3 g, dim3 b, cudaStream_t st) {
-        if (NR > 0) adjoint_fused_sweep<T, L, W, NR, NR != 0, 2><<<g, b, 0, st>>>(p);
-        else adjoint_fused_sweep<T, L, W, NR, false, 2><<<g, b, 0, st>>>(p);
-    }
-};
 
 template <typename T>
 History<T> make_history(const acf_batch *b) {
@@ -5598,7 +5387,8 @@ int adjoint_impl(acf_batch *b, const double *grad_rec, double *grad_src, double 
     if (A.grad_shell) ACF_CUDA(cudaMemsetAsync(A.grad_shell, 0, A.shell_total * sizeof(double), st));
     const LaunchShape L = single_shape(b);
     const LaunchShape LA = air ? single_shape(b, 2) : L;   // the air launches: 2 z elements each
-    const int64_t blocks = (int64_t)LA.grid.x * LA.grid.y * LA.grid.z;
+    const int64_t blocks = std::max((int64_t)LA.grid.x * LA.grid.y * LA.grid.z,
+                                    pack_adjoint_blocks<T>(make_room<T>(b, 0), b->planes, b->block_threads));
     const int NA = 3 * h.n_relax + 1;
     if (air) {
         if (A.air_blocks < blocks) {
@@ -5680,8 +5470,7 @@ int adjoint_impl(acf_batch *b, const double *grad_rec, double *grad_src, double 
                 return;
             }
         }
-        if (air) dispatch_pressure<T, AdjFusedAir>(h.has_layer, h.has_walls, h.n_relax, q, LA.grid, LA.block, s);
-        else dispatch_pressure<T, AdjFused>(h.has_layer, h.has_walls, h.n_relax, q, L.grid, L.block, s);
+        launch_pack_adjoint(q, h.has_layer, h.has_walls, h.n_relax, air, b->block_threads, s);
     };
     // Graph chunks of at most kAdjointChunk steps (one per segment when segments are shorter),
     // one graph per starting copy. Steps [e - G, e) in reverse: graph locals are captured in
@@ -5926,13 +5715,6 @@ struct BatchAdjPressure {
     }
 };
 
-template <typename T, bool L, bool W, int NR>
-struct BatchAdjFused {
-    static void launch(const BatchAdjointParams<T> &p, dim3 g, dim3 b, cudaStream_t st) {
-        adjoint_fused_batch<T, L, W, NR><<<g, b, 0, st>>>(p);
-    }
-};
-
 int batch_adjoint_prepare(acf_batch *b, int64_t max_steps) {
     if (!b) return fail(ACF_ERR_ARGUMENT, "null batch");
     if (max_steps < 1) return fail(ACF_ERR_ARGUMENT, "max_steps must be >= 1");
@@ -6129,9 +5911,13 @@ int batch_adjoint_impl(acf_batch *b, const double *grad_rec, double *grad_src, d
     for (int64_t t = n - 2; t >= 0; t--) {
         p.rooms = tables[parity];
         p.local_step = (int32_t)t;
-        dispatch_pressure<T, BatchAdjFused>(b->any_layer, b->any_walls, b->n_relax, p, grid, block, st);
+        p.tiles = b->pack_tiles;
+        p.n_tiles = b->n_pack_tiles;
+        launch_pack_adjoint_batch(p, b->any_layer, b->any_walls, b->n_relax, b->pack_ctas, st);
         parity ^= 1;
     }
+    p.tiles = b->tiles;
+    p.n_tiles = b->n_tiles;
     p.rooms = tables[parity];
     p.local_step = 0;
     if (b->any_layer) adjoint_velocity_batch<T, true><<<grid, block, 0, st>>>(p);

@@ -61,6 +61,17 @@ __device__ __forceinline__ Pack<float> pmul(const Pack<float> &x, float c) {
 __device__ __forceinline__ Pack<double> pmul(const Pack<double> &x, double c) {
     return {make_double2(x.a.x * c, x.a.y * c)};
 }
+__device__ __forceinline__ Pack<float> ptimes(const Pack<float> &x, const Pack<float> &y) {
+    return {mul2(x.a, y.a), mul2(x.b, y.b)};
+}
+__device__ __forceinline__ Pack<double> ptimes(const Pack<double> &x, const Pack<double> &y) {
+    return {make_double2(x.a.x * y.a.x, x.a.y * y.a.y)};
+}
+template <typename T>
+__device__ __forceinline__ Pack<T> zero_first(Pack<T> x) {
+    x.a.x = T(0);
+    return x;
+}
 template <typename T>
 __device__ __forceinline__ Pack<T> pzero() {
     if constexpr (sizeof(T) == 4) return {dup2(0.f), dup2(0.f)};
