@@ -8,10 +8,12 @@
 // (a sum, a smallest index) goes through distributed shared memory in a fixed order, so results do
 // not depend on timing and no scratch memory is needed. One CTA per channel left two thirds of the
 // SMs idle, read the signal up to three times with a stride and spent some 130 operations in double
-// precision on every level. 48 signals of 96,000 samples, cold caches: the curve 115 to 43 us (74 MB
-// of traffic, 11 us at the measured copy rate; bound now by double-precision issue and its phases'
-// barriers in two waves of CTAs), a clarity 19 to 14 us, the spectrum's peak 29 to 4 us, a fit 39
-// to 40 us (with the curve just written, in L2, 35 to 28).
+// precision on every level. 48 signals of 96,000 samples,
+// with the signal or curve in L2: the curve 113 to 37 us (74 MB of traffic, 11 us at the measured copy
+// rate; bound now by double-precision issue and its phases' barriers in two waves of CTAs), a fit 27 to
+// 23, a clarity 12 to 10; one signal 112 to 14, 26 to 13 and 12 to 7. From cold caches the spectrum's
+// peak takes 29 to 4 us. Signals of 600 samples pay for the cluster: a curve 4.3 to 6.2 us, a fit 6.2 to
+// 7.2.
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>

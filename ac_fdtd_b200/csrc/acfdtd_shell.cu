@@ -6,8 +6,7 @@
 // on the host took 2.1 ms for 128^3 and 9 ms for three rooms of 96 to 160 with 4 x 4 patches per wall,
 // a quarter of a gradient. Now (ms per gradient, before and after): 128^3 9.2 and 7.3, 101 x 86 x 92 with
 // air 5.5 and 4.7, the three rooms 34.2 and 25.5. The maps are 0.8 MB at 128^3; the launches take
-// microseconds, and what
-// is left is the copy to the caller.
+// microseconds, and what is left is the copy to the caller.
 
 #include "acfdtd_shell.cuh"
 
