@@ -42,11 +42,15 @@ __device__ __forceinline__ double block_sum(double v, double *shared) {
     for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
     if ((threadIdx.x & 31) == 0) shared[threadIdx.x >> 5] = v;
     __syncthreads();
-    double total = 0.0;
+    double level[kWarps];                        // pairwise: fewer roundings than one after the other
 #pragma unroll
-    for (int w = 0; w < kWarps; w++) total += shared[w];
+    for (int w = 0; w < kWarps; w++) level[w] = shared[w];
+#pragma unroll
+    for (int width = kWarps / 2; width > 0; width /= 2)
+#pragma unroll
+        for (int w = 0; w < width; w++) level[w] += level[w + width];
     __syncthreads();
-    return total;
+    return level[0];
 }
 
 __device__ __forceinline__ int64_t block_min(int64_t v, int64_t *shared) {
@@ -180,8 +184,9 @@ __device__ __forceinline__ Two cluster_sums(const cg::cluster_group &cluster, do
     b = block_sum(b, shared);
     if (threadIdx.x == 0) *mine = {a, b};
     gather(cluster, mine, all);
+    // from the last part on: a response decays, so its small sums come together before the large one
     Two total = {0.0, 0.0};
-    for (unsigned r = 0; r < cluster.num_blocks(); r++) {
+    for (int r = (int)cluster.num_blocks() - 1; r >= 0; r--) {
         total.a += all[r].a;
         total.b += all[r].b;
     }
