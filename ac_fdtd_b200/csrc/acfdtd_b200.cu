@@ -962,7 +962,7 @@ fused_staged_sweep(const StagedParams<T> g) {
 // ------------------------------------------------------------------------------------------
 // The fused step in single precision, lean in instructions (rooms with nz a multiple of 4).
 //
-// Bound by HBM only while its warps issue fast enough: fused_column spends about 190
+// Bound by HBM only while its warps issue fast enough: scalar code spends about 190
 // thread-instructions per cell, so under the power cap's lower SM clock the step slowed with the
 // clock. This column performs the same operations with a third of the instructions:
 //   * the two-lane f32x2 arithmetic of the staged sweep (same rounding, lane for lane);
@@ -995,7 +995,7 @@ struct LeanColumn {
 
 // ALIGNED: nz is a multiple of 4. Otherwise the last chunk of every row holds padding elements
 // (k >= nz), which this column leaves as they are, and the top face k = nz, which it damps
-// without a gradient update -- exactly as fused_column does -- with per-thread fix-ups that only
+// without a gradient update -- exactly as scalar code does -- with per-thread fix-ups that only
 // the threads of those chunks take.
 template <bool LAYER, bool ALIGNED>
 __device__ __forceinline__ LeanColumn lean_setup(const Room<float> &s, int j, int c) {
@@ -1023,7 +1023,7 @@ __device__ __forceinline__ LeanColumn lean_setup(const Room<float> &s, int j, in
         col.fj_cell = __ldg(s.cell[1] + j);
         col.fj_face = __ldg(s.face[1] + j);
         col.fj1_face = __ldg(s.face[1] + j + 1);
-        // padding lanes take the last cell's and the top face's factors, as fused_column does
+        // padding lanes take the last cell's and the top face's factors
         const int c_last = s.nz - 1, f_last = s.nz;
         auto kc = [&](int e) { return __ldg(s.cell[2] + (ALIGNED ? k0 + e : min(k0 + e, c_last))); };
         auto kf = [&](int e) { return __ldg(s.face[2] + (ALIGNED ? k0 + e : min(k0 + e, f_last))); };
@@ -2548,7 +2548,7 @@ __device__ __forceinline__ void lean_adjoint_column(const LeanAdjointParams &g, 
 }
 
 // The same step with the air-strength sums (relaxation states present): per-thread two-lane
-// sums over the launch's cells, then FP64 block sums into air_partials, as adjoint_fused_sweep.
+// sums over the launch's cells, then FP64 block sums into air_partials, as pack_adjoint.
 template <bool LAYER, bool WALLS, int NR>
 __global__ void __launch_bounds__(256, 2) lean_adjoint_air_sweep(const LeanAdjointParams g) {
     constexpr int NA = 3 * NR + 1;
