@@ -3,6 +3,10 @@
 // Faces on walls are not asked for (the pressure outside is the cell's own, a difference of zero:
 // neighbour offsets are 0 where the room ends, so no load is conditional), layer factors that are
 // exactly 1 are skipped, and a chunk that reaches past nz repeats its last real pressure.
+//
+// p, v and the relaxation states are read by plain loads: a step that was launched early is resident
+// while the step before still writes them, and the read-only path (__ldg) is for data that nothing
+// writes during the kernel. Layer profiles and wall pairs, written by the host alone, take that path.
 
 #ifndef ACFDTD_FUSED_KERNEL_CUH
 #define ACFDTD_FUSED_KERNEL_CUH
@@ -11,14 +15,6 @@
 
 namespace acf {
 namespace {
-
-__device__ __forceinline__ Pack<double> pack_ldg(const double *a) {
-    return {__ldg(reinterpret_cast<const double2 *>(a))};
-}
-__device__ __forceinline__ Pack<float> pack_ldg(const float *a) {
-    const float4 v = __ldg(reinterpret_cast<const float4 *>(a));
-    return {lo2(v), hi2(v)};
-}
 
 // One column of chunks over planes [i_begin, i_end). REC: also write the forward history.
 template <typename T, bool LAYER, bool WALLS, int NR, bool REC = false>
@@ -69,9 +65,9 @@ __device__ __forceinline__ void pack_column(const FusedParams<T> &f, int i_begin
     P pc, xl;
     {
         const int64_t base = (int64_t)i_begin * s.plane + column;
-        pc = pack_ldg(s.p + base);
-        const P below = pack_ldg(s.p + base - (i_begin > 0 ? s.plane : 0));
-        xl = moved(pack_ldg(s.vx + base), pc, below);
+        pc = pload(s.p + base);
+        const P below = pload(s.p + base - (i_begin > 0 ? s.plane : 0));
+        xl = moved(pload(s.vx + base), pc, below);
         if (tail) pc = mirrored(pc, real);
         if (LAYER) {
             const T fx = __ldg(s.face[0] + i_begin);
@@ -95,12 +91,12 @@ __device__ __forceinline__ void pack_column(const FusedParams<T> &f, int i_begin
             for (int r = 0; r < NR; r++) prefetch_l2(s.psi + r * s.field + next);
         }
         // ---- loads, all before the first store
-        P ph = pack_ldg(s.p + base + (inner ? s.plane : 0));
-        const P py_l = pack_ldg(s.p + base + y_lo), py_h = pack_ldg(s.p + base + y_hi);
-        P xh = pack_ldg(s.vx + base + s.plane), yl = pack_ldg(s.vy + base), yh = pack_ldg(s.vy + base + s.pz);
-        P zl = pack_ldg(s.vz + base);
-        const T pz_l = __ldg(s.p + base + z_lo), pz_h = __ldg(s.p + base + z_hi);
-        T za = k0 + W <= s.nz ? __ldg(s.vz + base + W) : T(0);
+        P ph = pload(s.p + base + (inner ? s.plane : 0));
+        const P py_l = pload(s.p + base + y_lo), py_h = pload(s.p + base + y_hi);
+        P xh = pload(s.vx + base + s.plane), yl = pload(s.vy + base), yh = pload(s.vy + base + s.pz);
+        P zl = pload(s.vz + base);
+        const T pz_l = s.p[base + z_lo], pz_h = s.p[base + z_hi];
+        T za = k0 + W <= s.nz ? s.vz[base + W] : T(0);
         P S[NR > 0 ? NR : 1];
 #pragma unroll
         for (int r = 0; r < NR; r++) S[r] = pload(s.psi + r * s.field + base);
