@@ -285,29 +285,8 @@ pack_adjoint(const __grid_constant__ AdjointParams<T> a) {
         pack_adjoint_column<T, LAYER, WALLS, NR, AIR>(a, i_begin, min(a.room.nx, i_begin + a.planes), j, c,
                                                       *a.step_base + a.local_step, acc);
     }
-    if (AIR) {                                   // the block's sums, and those over blocks and steps, in FP64
-        __shared__ double part[NA][kPackThreads / 32];
-        const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-        const int lane = tid & 31, warp = tid >> 5, warps = (blockDim.x * blockDim.y + 31) >> 5;
-        const int lanes = min(32, (int)(blockDim.x * blockDim.y) - 32 * warp);
-        const unsigned mask = lanes == 32 ? 0xffffffffu : (1u << lanes) - 1u;
-#pragma unroll
-        for (int t = 0; t < NA; t++) {
-            double v = total(acc[t]);
-            for (int o = 16; o > 0; o >>= 1) {
-                const double other = __shfl_down_sync(mask, v, o);
-                if (lane + o < lanes) v += other;
-            }
-            if (lane == 0) part[t][warp] = v;
-        }
-        __syncthreads();
-        if (tid < NA) {
-            double v = 0.0;
-            for (int w = 0; w < warps; w++) v += part[tid][w];
-            const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-            a.air_partials[block * NA + tid] += v;
-        }
-    }
+    if (AIR)                                     // uniform per launch: every thread reaches the barrier
+        add_block_sums<NA, kPackThreads>(a.air_partials, [&](int t) { return total(acc[t]); });
 }
 
 template <typename T, bool LAYER, bool WALLS, int NR>

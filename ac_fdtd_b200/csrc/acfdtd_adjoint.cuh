@@ -26,6 +26,32 @@ struct AdjointParams {
     T *out_vx, *out_vy, *out_vz, *out_d;
 };
 
+// The sums over a block of NA values per thread, sum(t) with t < NA, added to its partials in FP64. Blocks
+// of rooms that are narrow in y and z are smaller than a warp, and smaller than NA.
+template <int NA, int MAX_THREADS, typename F>
+__device__ __forceinline__ void add_block_sums(double *air_partials, F sum) {
+    __shared__ double part[NA][MAX_THREADS / 32];
+    const int threads = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + threadIdx.x;
+    const int lane = tid & 31, warp = tid >> 5, warps = (threads + 31) >> 5, lanes = min(32, threads - 32 * warp);
+    const unsigned mask = lanes == 32 ? 0xffffffffu : (1u << lanes) - 1u;
+#pragma unroll
+    for (int t = 0; t < NA; t++) {
+        double v = sum(t);
+        for (int o = 16; o > 0; o >>= 1) {
+            const double other = __shfl_down_sync(mask, v, o);
+            if (lane + o < lanes) v += other;
+        }
+        if (lane == 0) part[t][warp] = v;
+    }
+    __syncthreads();
+    const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    for (int t = tid; t < NA; t += threads) {
+        double v = 0.0;
+        for (int w = 0; w < warps; w++) v += part[t][w];
+        air_partials[block * NA + t] += v;
+    }
+}
+
 template <typename T>
 struct BatchAdjointParams {
     const AdjointParams<T> *rooms;

@@ -2245,25 +2245,8 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 8 ? (AIR && VW == kVec ? 1 
         adjoint_pressure_column<T, LAYER, WALLS, NR, AIR, VW>(a, i_begin, min(a.room.nx, i_begin + a.planes),
                                                                      j, c, *a.step_base + a.local_step, air_acc);
     }
-    if (AIR && NR > 0) {  // uniform per launch: every thread reaches the barrier
-        __shared__ double red[NA][8];
-        const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-        const int lane = tid & 31, warp = tid >> 5;
-        const int n_warps = (blockDim.x * blockDim.y + 31) >> 5;
-#pragma unroll
-        for (int t = 0; t < NA; t++) {
-            double v = (double)air_acc[t];
-            for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
-            if (lane == 0) red[t][warp] = v;
-        }
-        __syncthreads();
-        if (tid < NA) {
-            double v = 0.0;
-            for (int w = 0; w < n_warps; w++) v += red[tid][w];
-            const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-            a.air_partials[block * NA + tid] += v;
-        }
-    }
+    if constexpr (AIR && NR > 0)  // uniform per launch: every thread reaches the barrier
+        add_block_sums<NA, 256>(a.air_partials, [&](int t) { return (double)air_acc[t]; });
 }
 
 // The fused adjoint step in single precision for rooms with nz a multiple of 4 and no air
@@ -2563,23 +2546,7 @@ __global__ void __launch_bounds__(256, 2) lean_adjoint_air_sweep(const LeanAdjoi
         lean_adjoint_column<LAYER, WALLS, NR, true>(g, i_begin, min(a.room.nx, i_begin + a.planes), j, c,
                                                     *a.step_base + a.local_step, acc);
     }
-    __shared__ double red[NA][8];
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    const int lane = tid & 31, warp = tid >> 5;
-    const int n_warps = (blockDim.x * blockDim.y + 31) >> 5;
-#pragma unroll
-    for (int t = 0; t < NA; t++) {
-        double v = (double)acc[t].x + (double)acc[t].y;
-        for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
-        if (lane == 0) red[t][warp] = v;
-    }
-    __syncthreads();
-    if (tid < NA) {
-        double v = 0.0;
-        for (int w = 0; w < n_warps; w++) v += red[tid][w];
-        const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-        a.air_partials[block * NA + tid] += v;
-    }
+    add_block_sums<NA, 256>(a.air_partials, [&](int t) { return (double)acc[t].x + (double)acc[t].y; });
 }
 
 template <bool LAYER, bool WALLS, int NR>
