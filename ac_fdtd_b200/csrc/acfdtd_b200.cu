@@ -3899,6 +3899,30 @@ void launch_step(acf_batch *b, int32_t local, cudaStream_t st, cudaEvent_t *even
 // Steps from which a run takes the resident sweep, and the most of them in one launch.
 constexpr int64_t kResidentMinSteps = 8, kResidentMaxSteps = 2048;
 
+// Beyond 32 points every chunk scans every point at every step (column_points), so what counts is how many
+// chunks a thread has and how many threads there are. us per step with 40, 100 and 400 receivers, of the two
+// sweeps and of what would replace them: the resident sweep at 112^3 in single precision (four chunks per
+// thread) 34, 62, 206 and 36, 75, 269, at 96^3 in double precision 38, 64, 185 and 53, 110, 399, but at 64^3
+// (one chunk) 25, 44, 140 and 7, 13, 45, in double precision (two) 29, 49, 152 and 12, 25, 89; the fused step in
+// double precision, with twice the threads of the sweeps, at 144^3 130, 221, 676 and 113, 227, 797.
+// With 40 receivers three chunks (80^3 in double precision) take 26 against 33 us, and the fused step 39; at 96^3
+// it takes 39 against 38, at 112^3 53 against 62.
+constexpr int kFewPoints = 32;           // any step may have so many
+constexpr int kSomePoints = 64;          // resident threads of up to three chunks; fused steps in double precision
+                                         // of rooms from 0.3 of L2 on
+
+int64_t points_of(const RoomHost &h) { return h.n_src + h.n_rec; }
+
+bool resident_points(const acf_batch *b) {
+    const int64_t points = points_of(b->rooms[0]);
+    return points <= kFewPoints || b->resident.planes <= (points <= kSomePoints ? 3 : 2);
+}
+bool fused_points(const acf_batch *b) {
+    const int64_t points = points_of(b->rooms[0]);
+    return b->precision == 4 || points <= kFewPoints ||
+           (points <= kSomePoints && (double)b->room_block_bytes(0) >= 0.3 * (double)b->l2_bytes);
+}
+
 // Whether this run's steps go through the resident sweep: one room on the two-sweep or the fused
 // scheme, run in several steps per host call (a solver set to launch step by step, or timing its
 // sweeps, gets the sweeps it asked for), with a plan that fits the device and its inboxes in
@@ -3916,9 +3940,9 @@ bool resident_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
         cudaGetLastError();
         return false;
     }
-    if (b->resident_state > 0) return true;
-    b->resident_state = -1;
     const RoomHost &h = b->rooms[0];
+    if (b->resident_state > 0) return resident_points(b);
+    b->resident_state = -1;
     b->resident = resident_plan<T>(h.nx, h.ny, h.nz, h.n_relax, h.has_layer, b->sms, (size_t)b->smem_per_block);
     if (b->resident.planes == 0) return false;
     if (dev_malloc(&b->resident_mailbox, b->resident.mailbox_bytes) != cudaSuccess ||
@@ -3929,7 +3953,7 @@ bool resident_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
         return false;
     }
     b->resident_state = 1;
-    return true;
+    return resident_points(b);
 }
 
 // The whole run in launches of the resident sweep, in place in the current copy.
@@ -3974,6 +3998,7 @@ bool one_sweep_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
         b->rooms.size() != 1 || b->profiling || b->graph_steps == 0)
         return false;
     RoomHost &h = b->rooms[0];
+    if (!fused_points(b)) return false;
     if (b->precision == 4 && (double)b->room_block_bytes(0) < kOneSweepL2 * (double)b->l2_bytes) return false;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
@@ -4071,6 +4096,9 @@ int run_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st
         b->scheme = ACF_SCHEME_FUSED;
         n_steps -= last_in_place ? 1 : 0;
     }
+    // The fused scheme with many points in double precision: the sweeps, in place in the current copy.
+    if (b->scheme == ACF_SCHEME_FUSED && b->rooms.size() == 1 && !fused_points(b))
+        b->scheme = ACF_SCHEME_TWO_SWEEPS;
 
     int64_t done = 0;
     if (b->pressure_only() && b->po_first) {
@@ -4093,7 +4121,7 @@ int run_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st
             }
             b->graph_dirty = false;
         }
-        cudaGraphExec_t &exec = one_sweep ? b->graph_one : (fused && b->rooms[0].cur) ? b->graph_odd : b->graph;
+        cudaGraphExec_t &exec = one_sweep ? b->graph_one : b->rooms[0].cur ? b->graph_odd : b->graph;
         if (!exec) {
             if (!b->capture_stream)
                 ACF_CUDA(cudaStreamCreateWithFlags(&b->capture_stream, cudaStreamNonBlocking));
@@ -5296,7 +5324,12 @@ int forward_record_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cuda
     // One fused step per recorded step instead of two sweeps, into the second copy of p and v
     // (allocated here when the solver's scheme has none; two sweeps if that fails). Checkpoints
     // are copied from the primary copy at any step, so a run that keeps them stays in place.
-    const bool one_sweep = (!air || A.fields_recorded) && b->rooms[0].cur == 0 && make_second_copies(b, st);
+    // Many points are scanned by every chunk, and the chunk step is then the slower one (128^3 with air and 40
+    // receivers 78 against 61 us per step in single precision); the lean step is not.
+    const RoomHost &h = b->rooms[0];
+    const bool lean = sizeof(T) == 4 && h.nz % kVec == 0 && !A.fields_recorded;
+    const bool one_sweep = (!air || A.fields_recorded) && h.cur == 0 && (lean || points_of(h) <= kFewPoints) &&
+                           make_second_copies(b, st);
     const int mode = (A.fields_recorded ? 1 : 0) + (one_sweep ? 2 : 0);
     if (mode != A.direct_mode) {
         b->adj_graphs_dirty = true;           // the record graph holds the history pointers
@@ -5792,7 +5825,11 @@ int batch_forward_record_impl(acf_batch *b, int64_t n_steps, int64_t step_offset
     // Fused steps between the two copies of p and v; on the two-sweep scheme an odd last step is
     // the sweeps, in place, so that the state is in the rooms' own copies before and after. All
     // of them are the sweeps where the device has no room for second copies.
-    const bool one_sweep = make_second_copies(b, st);
+    // The sweeps also where rooms have many points (four rooms with 100 receivers each 230 against 259 us
+    // per step in single precision, 317 against 363 in double).
+    int64_t most_points = 0;
+    for (const RoomHost &h : b->rooms) most_points = std::max(most_points, points_of(h));
+    const bool one_sweep = (b->scheme == ACF_SCHEME_FUSED || most_points <= kSomePoints) && make_second_copies(b, st);
     if (one_sweep && b->room_table_dirty) {
         rc = upload_room_table<T>(b);
         if (rc) return rc;
