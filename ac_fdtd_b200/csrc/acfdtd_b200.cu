@@ -5302,6 +5302,22 @@ int record_steps(acf_batch *b, acf_batch::Graph &g, const void *state, const His
     return ACF_OK;
 }
 
+// Whether the recorded chunk step (into the second copy of p and v) is faster than the two recorded sweeps (in
+// place). With relaxation states it is not where the room in place stays in L2 and both copies do not, most
+// of all beside the history of D and psi; ragged rows lose from smaller sizes on. us per step of the sweeps
+// and of the chunk step, with that history, in single precision (both copies in parts of L2): 108^3 19.2 and
+// 17.4 (0.44), 112^3 20.4 and 24.6 (0.51), 128^3 24.7 and 37.0 (0.75), 152^3 60.8 and 66.9 (1.25), 160^3 73.8
+// and 73.3 (1.45), 176^3 96.6 and 84.1 (1.92); 93 x 91 x 95 15.8 and 14.5 (0.28), 97 x 131 x 77 17.8 and 18.9
+// (0.35), 150 x 130 x 171 62 and 62 (1.16), 165 x 171 x 163 87 and 79 (1.6); in double precision 92^3 23.2 and
+// 21.0 (0.55), 97 x 95 x 93 24.1 and 26.7 (0.60), 96^3 24.8 and 26.6 (0.65), 100^3 36.3 and 30.4 (0.71).
+bool chunk_record_faster(const acf_batch *b, bool fields) {
+    const RoomHost &h = b->rooms[0];
+    if (h.n_relax == 0) return true;
+    const double both = (double)(b->room_block_bytes(0) + (size_t)4 * h.field * b->elem()) / (double)b->l2_bytes;
+    if (b->precision == 8) return !fields || both < 0.58 || both > 0.68;
+    return both < (h.nz % kVec ? 0.33 : 0.48) || both > 1.3;
+}
+
 template <typename T>
 int forward_record_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st) {
     auto &A = b->adj;
@@ -5328,7 +5344,8 @@ int forward_record_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cuda
     // receivers 78 against 61 us per step in single precision); the lean step is not.
     const RoomHost &h = b->rooms[0];
     const bool lean = sizeof(T) == 4 && h.nz % kVec == 0 && !A.fields_recorded;
-    const bool one_sweep = (!air || A.fields_recorded) && h.cur == 0 && (lean || points_of(h) <= kFewPoints) &&
+    const bool one_sweep = (!air || A.fields_recorded) && h.cur == 0 &&
+                           (lean || (points_of(h) <= kFewPoints && chunk_record_faster(b, A.fields_recorded))) &&
                            make_second_copies(b, st);
     const int mode = (A.fields_recorded ? 1 : 0) + (one_sweep ? 2 : 0);
     if (mode != A.direct_mode) {
