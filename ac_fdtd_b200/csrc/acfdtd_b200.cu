@@ -4738,6 +4738,18 @@ void fused_slab_step(acf_batch *const *parts, int n, const int32_t *own_lo, cons
     for (int q = 0; q < n; q++) parts[q]->rooms[0].cur ^= 1;
 }
 
+// After the last step of parts on several GPUs: each part's stream waits for its neighbours', which store
+// into its ghost planes. Waiting for a part's own GPU then covers all that writes its memory, as closing
+// it (dev_free), reading its planes and reusing its blocks rely on.
+void wait_for_ghost_stores(acf_batch *const *parts, int n, const std::vector<cudaEvent_t> &done,
+                           const std::vector<cudaStream_t> &streams) {
+    for (int q = 0; q < n; q++) {
+        DeviceGuard g(parts[q]->device);
+        for (int r : {q - 1, q + 1})
+            if (r >= 0 && r < n) cudaStreamWaitEvent(streams[q], done[r], 0);
+    }
+}
+
 // Slab groups on the fused scheme: one launch per part and step. On one GPU the steps replay
 // from a CUDA graph of an even number of steps (the copies come back to the same parity);
 // across GPUs each part's step waits, by events, for its neighbours' previous step (which wrote
@@ -4805,6 +4817,7 @@ int run_fused_slabs(acf_batch *const *parts, int n, const int32_t *own_lo, const
         fused_slab_step<T>(parts, n, own_lo, own_hi, (int32_t)t, streams,
                            [&](int q) { cudaEventRecord(done_ev[q], streams[q]); });
     }
+    wait_for_ghost_stores(parts, n, done_ev, streams);
     const cudaError_t e = cudaGetLastError();
     release();
     if (e != cudaSuccess) return fail(ACF_ERR_CUDA, "slab step: %s", cudaGetErrorString(e));
@@ -4898,6 +4911,7 @@ int run_slabs_impl(acf_batch *const *parts, int n, const int32_t *own_lo, const 
             parts[q]->launches += 2;
         }
     }
+    if (!one_device) wait_for_ghost_stores(parts, n, pres_done, streams);
     const cudaError_t e = cudaGetLastError();
     release();
     if (e != cudaSuccess) return fail(ACF_ERR_CUDA, "slab step: %s", cudaGetErrorString(e));

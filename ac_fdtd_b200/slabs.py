@@ -328,6 +328,10 @@ class SlabGroup(_SlabSet):
             if self._receivers else np.zeros((0, self.step_index), dtype=self.slabs[0].dtype)
 
     def close(self) -> None:
+        if self._several_devices:
+            # A part's memory goes to the next solver of its GPU, and its neighbours' GPUs store into
+            # its ghost planes: nothing of any part may be in flight when the first one closes.
+            self.synchronize()
         for s in self.slabs:
             s.close()
 
