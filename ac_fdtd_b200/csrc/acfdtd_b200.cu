@@ -3217,7 +3217,7 @@ struct acf_batch {
     float *psi2 = nullptr;
 
     // Rooms held on chip (acfdtd_resident.cuh): how the room is cut, found at the first run that
-    // asks (resident_state 0 until then; 1 usable, -1 not), the neighbours' inboxes and tags.
+    // asks (resident_state 0 until then; 1 if it can be, -1 not), the neighbours' inboxes and tags.
     int resident_state = 0;
     ResidentPlan resident;
     void *resident_mailbox = nullptr;
@@ -3923,12 +3923,45 @@ bool fused_points(const acf_batch *b) {
            (points <= kSomePoints && (double)b->room_block_bytes(0) >= 0.3 * (double)b->l2_bytes);
 }
 
+// Whether the resident sweep is faster than the step that would run instead. Up to three x planes per thread
+// it is, two to six times. With four its threads share a scheduler's issue slots four ways, and a layer with
+// relaxation states spills them to local memory; with six and eight it has two barriers per step and leaves
+// what does not fit (a relaxation state) in L2. us per step, resident and the other:
+//   the lean step (fused, single precision), four planes: 98^3 walls and air 8.4 and 11.4, with a layer 13.8
+//     and 12.3, at 384 threads (96^3) 10.0 and 10.9; four states 13.4 and 12.6; 100^3 layer and walls 8.1 and
+//     10.4, layer alone 9.2 and 8.2. Six: walls 104^3 8.4 and 9.4, 116^3 9.8 and 10.6; with air 104^3 11.5 and
+//     10.9, 116^3 15.6 and 13.4, and with a layer 108^3 17.5 and 12.6. Eight: walls 120^3 11.7 and 10.6, 128^3
+//     12.2 and 12.4.
+//   the two sweeps in single precision, six: 112^3 with air 13.8 and 16.4, 108^3 four states 17.7 and 16.6 (a
+//     layer too, at 104^3, 19.5 and 18.6), 116^3 (480 threads) a layer alone 15.6 and 15.1; eight: 128^3 walls 12.1 and 14.8, with a layer
+//     too 17.0 and 18.9, a layer alone 20.1 and 16.3, 112 x 113 x 114 with air 18.7 and 17.0.
+//   the chunk step in double precision, four: 80^3 walls and air 8.4 and 11.1, with a layer 14.3 and 13.5; six:
+//     88^3 13.0 and 15.6, with a layer 17.2 and 19.5, 86^3 a layer alone 14.7 and 13.4, 84^3 with four states
+//     15.5 and 13.5; eight: 96^3 walls 12.2 and 11.2, a layer too 17.5 and 16.7, 92^3 with air 17.5 and 16.9.
+bool resident_faster(const acf_batch *b) {
+    const RoomHost &h = b->rooms[0];
+    const int planes = b->resident.planes, threads = b->resident.threads, states = h.n_relax;
+    const bool layer = h.has_layer;
+    if (planes <= 3) return true;
+    if (b->precision == 8) {
+        if (planes == 4) return !layer || states < 3;
+        return planes == 6 && states < 4 && (!layer || h.has_walls || states > 0);
+    }
+    if (b->scheme == ACF_SCHEME_FUSED) {
+        if (planes == 4) return !layer || threads < 384 || (threads == 384 && states < 4) || (states == 0 && h.has_walls);
+        return planes == 6 && states == 0 && !layer;
+    }
+    if (planes == 4) return true;
+    if (planes == 6) return states < 4 && (!layer || h.has_walls || states > 0 || threads <= 448);
+    return states == 0 && (!layer || h.has_walls);
+}
+
 // Whether this run's steps go through the resident sweep: one room on the two-sweep or the fused
 // scheme, run in several steps per host call (a solver set to launch step by step, or timing its
-// sweeps, gets the sweeps it asked for), with a plan that fits the device and its inboxes in
-// place. They are allocated here, once per handle; where that fails, and inside a stream capture,
-// the sweeps are used as they are without it. Eight steps: loading and storing the state costs
-// as much as two steps of the sweeps.
+// sweeps, gets the sweeps it asked for), with a plan that fits the device, is faster, and has its
+// inboxes in place. They are allocated at the first such run, once per handle; where that fails, and
+// inside a stream capture, the sweeps are used as they are without it. Eight steps: loading and storing
+// the state costs as much as two steps of the sweeps.
 template <typename T>
 bool resident_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
     if (b->resident_state < 0 || n_steps < kResidentMinSteps || b->rooms.size() != 1 || b->profiling ||
@@ -3941,19 +3974,21 @@ bool resident_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
         return false;
     }
     const RoomHost &h = b->rooms[0];
-    if (b->resident_state > 0) return resident_points(b);
-    b->resident_state = -1;
-    b->resident = resident_plan<T>(h.nx, h.ny, h.nz, h.n_relax, h.has_layer, b->sms, (size_t)b->smem_per_block);
-    if (b->resident.planes == 0) return false;
+    if (b->resident_state == 0) {
+        b->resident = resident_plan<T>(h.nx, h.ny, h.nz, h.n_relax, h.has_layer, b->sms, (size_t)b->smem_per_block);
+        b->resident_state = b->resident.planes == 0 ? -1 : 1;
+    }
+    if (b->resident_state < 0 || !resident_points(b) || !resident_faster(b)) return false;
+    if (b->resident_epoch) return true;
     if (dev_malloc(&b->resident_mailbox, b->resident.mailbox_bytes) != cudaSuccess ||
         dev_malloc(&b->resident_epoch, 2 * sizeof(uint32_t)) != cudaSuccess ||
         cudaMemsetAsync(b->resident_mailbox, 0, b->resident.mailbox_bytes, st) != cudaSuccess ||
         cudaMemsetAsync(b->resident_epoch, 0, 2 * sizeof(uint32_t), st) != cudaSuccess) {
         cudaGetLastError();
+        b->resident_state = -1;
         return false;
     }
-    b->resident_state = 1;
-    return resident_points(b);
+    return true;
 }
 
 // The whole run in launches of the resident sweep, in place in the current copy.
