@@ -3150,7 +3150,7 @@ struct acf_batch {
 
     void *state = nullptr;           // every room's fields, one arena
     size_t state_bytes = 0;
-    void *room_table = nullptr;      // device array of Room<T>, one per room
+    void *room_table = nullptr;      // device array of Room<T>: one per room and parity
     void *fused_table = nullptr;     // fused scheme on a batch: 2 x rooms FusedParams<T>, by parity
     bool room_table_dirty = true;
     Tile *tiles = nullptr;
@@ -3397,36 +3397,61 @@ bool make_second_copies(acf_batch *b, cudaStream_t st) {
     return true;
 }
 
+// Both parities: entry [parity * rooms + r] of the tables reads the copy that is current at that parity.
 template <typename T>
 int upload_room_table(acf_batch *b) {
-    std::vector<Room<T>> table(b->rooms.size());
-    for (size_t r = 0; r < b->rooms.size(); r++) table[r] = make_room<T>(b, (int)r);
-    if (!b->room_table) ACF_CUDA(dev_malloc(&b->room_table, table.size() * sizeof(Room<T>)));
-    ACF_CUDA(cudaMemcpy(b->room_table, table.data(), table.size() * sizeof(Room<T>), cudaMemcpyHostToDevice));
-    if (second_copies(b)) {
-        // Both parities: entry [parity * rooms + r] reads the copy that is current at that parity.
-        const size_t n = b->rooms.size();
-        std::vector<FusedParams<T>> fused(2 * n);
-        for (int parity = 0; parity < 2; parity++)
-            for (size_t r = 0; r < n; r++) {
-                RoomHost &h = b->rooms[r];
-                const int saved = h.cur;
-                h.cur = parity;
+    const size_t n = b->rooms.size();
+    const bool both = second_copies(b);
+    std::vector<Room<T>> table(2 * n);
+    std::vector<FusedParams<T>> fused(both ? 2 * n : 0);
+    for (int parity = 0; parity < (both ? 2 : 1); parity++)
+        for (size_t r = 0; r < n; r++) {
+            RoomHost &h = b->rooms[r];
+            const int saved = h.cur;
+            h.cur = parity;
+            table[parity * n + r] = make_room<T>(b, (int)r);
+            if (both) {
                 FusedParams<T> &f = fused[parity * n + r];
                 f = FusedParams<T>{};
-                f.room = make_room<T>(b, (int)r);
+                f.room = table[parity * n + r];
                 f.np = (T *)b->other_ptr((int)r, ACF_FIELD_P);
                 f.nvx = (T *)b->other_ptr((int)r, ACF_FIELD_VX);
                 f.nvy = (T *)b->other_ptr((int)r, ACF_FIELD_VY);
                 f.nvz = (T *)b->other_ptr((int)r, ACF_FIELD_VZ);
-                h.cur = saved;
             }
+            h.cur = saved;
+        }
+    if (!b->room_table) ACF_CUDA(dev_malloc(&b->room_table, table.size() * sizeof(Room<T>)));
+    ACF_CUDA(cudaMemcpy(b->room_table, table.data(), table.size() * sizeof(Room<T>), cudaMemcpyHostToDevice));
+    if (both) {
         if (!b->fused_table) ACF_CUDA(dev_malloc(&b->fused_table, fused.size() * sizeof(FusedParams<T>)));
         ACF_CUDA(cudaMemcpy(b->fused_table, fused.data(), fused.size() * sizeof(FusedParams<T>),
                             cudaMemcpyHostToDevice));
     }
     b->room_table_dirty = false;
     return ACF_OK;
+}
+
+// The rooms at the copy that is current, for the sweeps in place.
+template <typename T>
+const Room<T> *current_rooms(const acf_batch *b) {
+    return (const Room<T> *)b->room_table + (b->rooms[0].cur ? b->rooms.size() : 0);
+}
+
+// Whether a batch on the fused scheme in single precision takes the two sweeps, in place in the current copy:
+// where the rooms in place stay in L2 and both their copies do not. us per step of the sweeps and of the fused step
+// (both copies in parts of L2), with air: 2 x 102^3 28 and 29 (0.73), 2 x 104^3 28 and 34 (0.82), 4 of 60 to 110 34
+// and 44 (0.98), 6 x 76^3 35 and 47 (0.96), 2 x 120^3 46 and 48 (1.24), 2 x 100^3 28.4 and 27.5 (0.70), 40 x 44^3 60
+// and 58 (1.29); without relaxation states 2 x 116^3 29 and 30 (0.79), 2 x 120^3 27 and 30 (0.90), 2 x 112^3 25.0 and
+// 24.8 (0.74), 2 x 122^3 42 and 37 (0.93). In double precision the fused step is the faster one throughout (2 x 92^3
+// 45 and 41, 2 x 128^3 128 and 93).
+bool batch_sweeps_faster(const acf_batch *b) {
+    if (b->precision == 8 || b->rooms.size() < 2) return false;
+    double bytes = 0.0;
+    for (size_t r = 0; r < b->rooms.size(); r++)
+        bytes += (double)(b->room_block_bytes((int)r) + (size_t)4 * b->rooms[r].field * b->elem());
+    const double both = bytes / (double)b->l2_bytes;
+    return b->n_relax > 0 ? both > 0.72 && both < 1.25 : both > 0.77 && both < 0.92;
 }
 
 // Tiles in room order, then plane group, then (row, chunk) block: neighbouring tiles of one
@@ -3882,7 +3907,7 @@ void launch_step(acf_batch *b, int32_t local, cudaStream_t st, cudaEvent_t *even
                                              L.block, st);
     } else {
         BatchParams<T> p{};
-        p.rooms = (const Room<T> *)b->room_table;
+        p.rooms = current_rooms<T>(b);
         p.tiles = b->tiles;
         p.n_tiles = b->n_tiles;
         p.local_step = local;
@@ -4131,8 +4156,8 @@ int run_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st
         b->scheme = ACF_SCHEME_FUSED;
         n_steps -= last_in_place ? 1 : 0;
     }
-    // The fused scheme with many points in double precision: the sweeps, in place in the current copy.
-    if (b->scheme == ACF_SCHEME_FUSED && b->rooms.size() == 1 && !fused_points(b))
+    // The fused scheme where the sweeps are faster: in place in the current copy.
+    if (b->scheme == ACF_SCHEME_FUSED && (b->rooms.size() == 1 ? !fused_points(b) : batch_sweeps_faster(b)))
         b->scheme = ACF_SCHEME_TWO_SWEEPS;
 
     int64_t done = 0;
@@ -5895,7 +5920,8 @@ int batch_forward_record_impl(acf_batch *b, int64_t n_steps, int64_t step_offset
     // per step in single precision, 317 against 363 in double).
     int64_t most_points = 0;
     for (const RoomHost &h : b->rooms) most_points = std::max(most_points, points_of(h));
-    const bool one_sweep = (b->scheme == ACF_SCHEME_FUSED || most_points <= kSomePoints) && make_second_copies(b, st);
+    const bool one_sweep = !batch_sweeps_faster(b) && (b->scheme == ACF_SCHEME_FUSED || most_points <= kSomePoints) &&
+                           make_second_copies(b, st);
     if (one_sweep && b->room_table_dirty) {
         rc = upload_room_table<T>(b);
         if (rc) return rc;
@@ -5910,7 +5936,7 @@ int batch_forward_record_impl(acf_batch *b, int64_t n_steps, int64_t step_offset
         for (RoomHost &h : b->rooms) h.cur ^= 1;
     }
     BatchParams<T> v{};
-    v.rooms = (const Room<T> *)b->room_table;
+    v.rooms = current_rooms<T>(b);
     v.tiles = b->tiles;
     v.n_tiles = b->n_tiles;
     v.step_base = b->step_base;
