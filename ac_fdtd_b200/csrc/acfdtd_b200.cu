@@ -4016,9 +4016,11 @@ bool resident_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
     return true;
 }
 
-// The whole run in launches of the resident sweep, in place in the current copy.
+// The run in launches of the resident sweep, in place in the current copy; the steps taken. They are
+// fewer than `n_steps` where the device refuses a cooperative launch (it cannot have all its CTAs resident, for
+// what else holds the SMs): the handle then uses the sweeps, from the next step on.
 template <typename T>
-int run_resident(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st) {
+int64_t run_resident(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st) {
     const RoomHost &h = b->rooms[0];
     ResidentRun<T> run;
     run.room = make_room<T>(b, 0);
@@ -4030,16 +4032,22 @@ int run_resident(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_
     run.epoch = b->resident_epoch;
     run.wait_limit_ns = b->test_wait_limit_ns ? b->test_wait_limit_ns : kWaitLimitNs;
     run.stop_step = b->test_skip_plane;
-    for (int64_t done = 0; done < n_steps;) {
+    const char *inject = getenv("ACF_INJECT_LAUNCH_REFUSAL");
+    const bool refused = inject && *inject && strcmp(inject, "0") != 0;
+    int64_t done = 0;
+    while (done < n_steps) {
         int64_t n = std::min(kResidentMaxSteps, n_steps - done);
         if (n_steps - done - n == 1) n -= 1;      // a launch takes two steps or more
         run.steps = (int)n;
-        ACF_CUDA(resident_launch<T>(b->resident, run, step_offset + done, st));
+        if (refused || resident_launch<T>(b->resident, run, step_offset + done, st) != cudaSuccess) {
+            cudaGetLastError();
+            b->resident_state = -1;
+            break;
+        }
         b->launches += 2;
         done += n;
     }
-    ACF_CUDA(cudaGetLastError());
-    return ACF_OK;
+    return done;
 }
 
 // Whether a run of the two-sweep scheme takes its steps in pairs of fused steps, which end in the
@@ -4083,7 +4091,15 @@ bool one_sweep_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
 
 template <typename T>
 int run_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st) {
-    if (resident_ready<T>(b, n_steps, st)) return run_resident<T>(b, n_steps, step_offset, st);
+    if (resident_ready<T>(b, n_steps, st)) {
+        const int64_t done = run_resident<T>(b, n_steps, step_offset, st);
+        if (done == n_steps) {
+            ACF_CUDA(cudaGetLastError());
+            return ACF_OK;
+        }
+        n_steps -= done;
+        step_offset += done;
+    }
     if (b->rooms.size() > 1 && b->room_table_dirty) {
         int rc = upload_room_table<T>(b);
         if (rc) return rc;

@@ -229,8 +229,9 @@ int acf_set_wait_test(acf_solver *solver, int64_t wait_limit_ns, int32_t skip_pl
  * itself. Otherwise a single room on the two-sweep or fused scheme whose state fits the GPU's
  * registers and shared memory (up to about 2 million cells in single precision, 900 thousand in
  * double; fewer with relaxation states) takes runs of 8 steps or more in one cooperative launch
- * per 2048 steps, with the same results bit for bit; its inboxes (at most 20 MB) are allocated at
- * the first such run, and where that fails, or inside a stream capture, the sweeps are used. */
+ * per 2048 steps where that is faster, with the same results bit for bit; its inboxes (at most 20 MB) are
+ * allocated at the first such run, and where that fails, where the device refuses the launch, or
+ * inside a stream capture, the sweeps are used. */
 int acf_set_graph(acf_solver *solver, int32_t steps_per_graph);
 
 /* Launch geometry of both sweeps: threads per block (power of two, 32..256) and consecutive
