@@ -20,7 +20,7 @@ from .grid import Grid, max_stable_time_step
 from .io import resample, write_wav
 from .medium import AIR, Medium
 from .room import ImpulseResponse, Room, simulate_impulse_response
-from .solver import CudaAcousticFDTD, pinned_array
+from .solver import CudaAcousticFDTD, pinned_array, release_memory
 from .sources import band_limited_impulse, deconvolve, gaussian_derivative_pulse, gaussian_pulse
 
 AcousticFDTD = CudaAcousticFDTD
@@ -47,6 +47,7 @@ __all__ = [
     "max_stable_time_step",
     "pinned_array",
     "reflection_coefficient",
+    "release_memory",
     "resample",
     "simulate_impulse_response",
     "write_wav",

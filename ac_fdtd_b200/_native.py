@@ -46,6 +46,7 @@ EXPORTED_SYMBOLS = (
     "acf_set_wait_test", "acf_schroeder_decay", "acf_decay_fit", "acf_clarity",
     "acf_spectral_divide", "acf_pressure_only_energy_terms", "acf_set_time_blocking",
     "acf_get_time_blocking", "acf_adjoint_wall_gradients", "acf_batch_adjoint_wall_gradients",
+    "acf_release_memory",
 )
 
 SCHEME_TWO_SWEEPS, SCHEME_FUSED, SCHEME_FUSED_STAGED, SCHEME_PRESSURE_ONLY = 0, 1, 2, 3
@@ -107,6 +108,7 @@ _SIGNATURES = {
     "acf_profile_read": (ctypes.c_int, [_P, _DP, _DP, _I64P]),
     "acf_launch_count": (ctypes.c_int64, [_P]),
     "acf_synchronize": (ctypes.c_int, [_P]),
+    "acf_release_memory": (ctypes.c_int, []),
     "acf_host_alloc": (ctypes.c_int, [ctypes.c_size_t, ctypes.POINTER(_P)]),
     "acf_host_free": (ctypes.c_int, [_P]),
     "acf_energy_terms_noalloc": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_int32, ctypes.c_int32,

@@ -49,6 +49,7 @@
 #include <mutex>
 #include <new>
 #include <unordered_map>
+#include <unordered_set>
 #include <vector>
 
 #include "acfdtd_b200.h"
@@ -2947,8 +2948,10 @@ struct DeviceGuard {
 // position, a sweep over designs) otherwise pays cudaMalloc and cudaFree (350 to 700 us each here,
 // 20 of them per solver) and a pinned word (3 ms) more than for the run: blocks given back are kept
 // for the next handle of this process, at most kCacheBytes of them in all (the oldest go first), and
-// every one is freed before an allocation is reported as failed. A block is given back only
-// once the device is idle, as cudaFree itself waits, so the next owner may use it on any stream.
+// every one is freed before an allocation is reported as failed, and so are second copies of p and v that their
+// handle can do without (SecondUse); acf_release_memory frees both at once, for other allocators of the process. A
+// block is given back only once the device is idle, as cudaFree itself waits, so the next owner may use
+// it on any stream.
 constexpr size_t kCacheBytes = (size_t)256 << 20;
 
 struct BlockCache {
@@ -2961,6 +2964,7 @@ struct BlockCache {
     std::unordered_map<void *, Block> used;
     std::deque<Block> idle;        // oldest first
     size_t idle_bytes = 0;
+    std::unordered_set<acf_batch *> spare;       // handles whose second copies no call is using
 
     // Free idle blocks, oldest first, until at most `keep` bytes remain.
     void trim(size_t keep) {
@@ -2978,6 +2982,8 @@ BlockCache &block_cache() {
     static BlockCache *cache = new BlockCache;   // outlives every handle, also at process exit
     return *cache;
 }
+
+void free_spare_copies(BlockCache &cache, int device);
 
 cudaError_t dev_malloc_bytes(void **out, size_t bytes) {
     BlockCache &cache = block_cache();
@@ -3004,6 +3010,11 @@ cudaError_t dev_malloc_bytes(void **out, size_t bytes) {
         if (err == cudaErrorMemoryAllocation && cache.idle_bytes > 0) {
             cudaGetLastError();
             cache.trim(0);
+            err = cudaMalloc(&block.pointer, bytes);
+        }
+        if (err == cudaErrorMemoryAllocation && !cache.spare.empty()) {
+            cudaGetLastError();
+            free_spare_copies(cache, device);
             err = cudaMalloc(&block.pointer, bytes);
         }
         if (err != cudaSuccess) return err;
@@ -3181,6 +3192,7 @@ struct acf_batch {
     cudaGraphExec_t graph = nullptr, graph_odd = nullptr;
     cudaGraphExec_t graph_one = nullptr;   // the two-sweep scheme's steps as fused steps (one_sweep)
     int one_sweep_state = 0;               // 0 undecided, 1 the second copy is there, -1 not
+    bool second_gone = false;              // its second copies were freed while it did not use them
     cudaStream_t capture_stream = nullptr;
     bool graph_dirty = true;
 
@@ -3380,12 +3392,77 @@ bool second_copies(const acf_batch *b) {
     return true;
 }
 
+size_t second_bytes(const acf_batch *b, const RoomHost &h) { return ((size_t)4 * h.field + (size_t)h.pz) * b->elem(); }
+
+// A call that uses a handle's second copies, or may. Between such calls the two-sweep scheme can do without
+// them: an allocation that would fail frees them, and the next run that wants them allocates them anew.
+struct SecondUse {
+    acf_batch *b;
+    explicit SecondUse(acf_batch *handle) : b(handle) {
+        std::lock_guard<std::mutex> hold(block_cache().lock);
+        block_cache().spare.erase(b);
+        if (!b->second_gone) return;
+        b->second_gone = false;
+        b->one_sweep_state = 0;
+        b->graph_dirty = b->adj_graphs_dirty = b->room_table_dirty = true;
+    }
+    ~SecondUse() {
+        if (b->scheme != ACF_SCHEME_TWO_SWEEPS) return;
+        bool any = false;
+        for (const RoomHost &h : b->rooms) {
+            if (h.cur) return;
+            any = any || h.second;
+        }
+        if (!any) return;
+        std::lock_guard<std::mutex> hold(block_cache().lock);
+        block_cache().spare.insert(b);
+    }
+    SecondUse(const SecondUse &) = delete;
+};
+
+// With the cache's lock held: the second copies that nothing uses, on one device or (-1) on all.
+void free_spare_copies(BlockCache &cache, int device) {
+    for (auto at = cache.spare.begin(); at != cache.spare.end();) {
+        acf_batch *b = *at;
+        if (device >= 0 && b->device != device) {
+            ++at;
+            continue;
+        }
+        DeviceGuard guard(b->device);
+        if (cudaDeviceSynchronize() != cudaSuccess) {      // what was queued with them
+            cudaGetLastError();
+            ++at;
+            continue;
+        }
+        for (RoomHost &h : b->rooms) {
+            if (!h.second) continue;
+            cache.used.erase(h.second);
+            cudaFree(h.second);
+            h.second = nullptr;
+        }
+        b->second_gone = true;
+        at = cache.spare.erase(at);
+    }
+}
+
+// Device memory that allocations of this library can have: free, idle in the cache, or spare.
+size_t obtainable_bytes(int device, size_t free_bytes) {
+    BlockCache &cache = block_cache();
+    std::lock_guard<std::mutex> hold(cache.lock);
+    for (const BlockCache::Block &idle : cache.idle)
+        if (idle.device == device) free_bytes += idle.bytes;
+    for (const acf_batch *b : cache.spare)
+        for (const RoomHost &h : b->rooms)
+            if (b->device == device && h.second) free_bytes += second_bytes(b, h);
+    return free_bytes;
+}
+
 // The second copies of p and v of the rooms that have none, zeroed on `st`; false when the device
 // has no room for one of them (those already there stay).
 bool make_second_copies(acf_batch *b, cudaStream_t st) {
     for (RoomHost &h : b->rooms) {
         if (h.second) continue;
-        const size_t bytes = ((size_t)4 * h.field + (size_t)h.pz) * b->elem();
+        const size_t bytes = second_bytes(b, h);
         if (dev_malloc(&h.second, bytes) != cudaSuccess) {
             cudaGetLastError();
             h.second = nullptr;
@@ -4076,7 +4153,7 @@ bool one_sweep_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
     if (b->one_sweep_state == 0) {
         b->one_sweep_state = -1;
         if (!h.second) {
-            const size_t bytes = ((size_t)4 * h.field + (size_t)h.pz) * b->elem();
+            const size_t bytes = second_bytes(b, h);
             size_t free_bytes = 0, total_bytes = 0;
             if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess || bytes > free_bytes / 16) {
                 cudaGetLastError();
@@ -4091,6 +4168,7 @@ bool one_sweep_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
 
 template <typename T>
 int run_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st) {
+    const SecondUse use(b);
     if (resident_ready<T>(b, n_steps, st)) {
         const int64_t done = run_resident<T>(b, n_steps, step_offset, st);
         if (done == n_steps) {
@@ -4316,6 +4394,10 @@ void free_room(RoomHost &h) {
 void free_batch(acf_batch *b) {
     if (!b) return;
     DeviceGuard guard(b->device);
+    {
+        std::lock_guard<std::mutex> hold(block_cache().lock);
+        block_cache().spare.erase(b);
+    }
     cudaDeviceSynchronize();       // nothing of this handle is in flight when its memory goes
     if (b->graph) cudaGraphExecDestroy(b->graph);
     if (b->graph_odd) cudaGraphExecDestroy(b->graph_odd);
@@ -5170,10 +5252,11 @@ int set_scheme(acf_batch *b, int32_t scheme) {
                         b->staged_rows, b->staged_stages);
     }
     DeviceGuard guard(b->device);
+    const SecondUse use(b);
     if (scheme != ACF_SCHEME_TWO_SWEEPS) {
         for (RoomHost &h : b->rooms) {
             if (h.second) continue;
-            const size_t bytes = ((size_t)4 * h.field + (size_t)h.pz) * b->elem();
+            const size_t bytes = second_bytes(b, h);
             if (dev_malloc(&h.second, bytes) != cudaSuccess)
                 return fail(ACF_ERR_MEMORY, "cudaMalloc of %zu bytes for the fused scheme failed", bytes);
             ACF_CUDA(cudaMemset(h.second, 0, bytes));
@@ -5410,6 +5493,7 @@ bool chunk_record_faster(const acf_batch *b, bool fields) {
 
 template <typename T>
 int forward_record_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st) {
+    const SecondUse use(b);
     auto &A = b->adj;
     if (A.step0 != step_offset) b->adj_graphs_dirty = true;
     A.recorded = n_steps;
@@ -5690,11 +5774,7 @@ int adjoint_prepare(acf_batch *b, int32_t flags, int64_t max_steps, int32_t ever
         const double whole = (double)max_steps * (1 + h.n_relax) * h.field * b->elem();
         size_t free_bytes = 0, total_bytes = 0;
         ACF_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
-        {                          // idle blocks of the cache are given back before an allocation fails
-            std::lock_guard<std::mutex> hold(block_cache().lock);
-            for (const BlockCache::Block &idle : block_cache().idle)
-                if (idle.device == b->device) free_bytes += idle.bytes;
-        }
+        free_bytes = obtainable_bytes(b->device, free_bytes);
         every = whole <= 0.6 * (double)free_bytes ? (int32_t)std::min<int64_t>(max_steps, INT32_MAX)
                                                    : (int32_t)std::ceil(std::sqrt((double)max_steps));
     }
@@ -5921,6 +6001,7 @@ int upload_adjoint_table(acf_batch *b, int64_t n) {
 
 template <typename T>
 int batch_forward_record_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st) {
+    const SecondUse use(b);
     b->badj_step0 = step_offset;
     b->badj_recorded = n_steps;
     if (b->room_table_dirty) {
@@ -6631,6 +6712,13 @@ int acf_energy_terms_noalloc(const void *p, const void *vx, const void *vy, cons
                                                            nx, ny, nz, inv_dx, scratch);
     energy_finish<<<1, 32, 0, st>>>(scratch, nx + 1, terms_device);
     ACF_CUDA(cudaGetLastError());
+    return ACF_OK;
+}
+
+int acf_release_memory(void) {
+    std::lock_guard<std::mutex> hold(block_cache().lock);
+    block_cache().trim(0);
+    free_spare_copies(block_cache(), -1);
     return ACF_OK;
 }
 

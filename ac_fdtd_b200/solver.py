@@ -23,7 +23,7 @@ from .coefficients import room_coefficients
 from .grid import cell_index
 from .medium import AIR
 
-__all__ = ["CudaAcousticFDTD", "DEFAULT_STEPS_PER_GRAPH", "pinned_array"]
+__all__ = ["CudaAcousticFDTD", "DEFAULT_STEPS_PER_GRAPH", "pinned_array", "release_memory"]
 
 #: Steps captured per CUDA graph for long runs; shorter runs launch step by step. A room small
 #: enough for the GPU's registers and shared memory takes many steps per launch instead (0 turns
@@ -118,6 +118,13 @@ def pinned_array(shape, dtype=np.float32) -> np.ndarray:
     array = np.asarray(_PinnedBlock(_native.library(), tuple(shape), np.dtype(dtype)))
     array[...] = 0
     return array
+
+
+def release_memory() -> None:
+    """Give back the device memory that the library holds without needing it (``acf_release_memory``): blocks
+    of closed solvers kept for the next ones, and second copies that open ones can do without. For
+    other allocators of the process; the library's own allocations do this before they fail."""
+    _native.check(_native.library().acf_release_memory(), "acf_release_memory")
 
 
 class CudaAcousticFDTD:

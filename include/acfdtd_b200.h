@@ -457,6 +457,13 @@ int acf_batch_set_coefficients(acf_batch *batch, int32_t room, const acf_config 
 /* Block until all work queued on `stream` is done. */
 int acf_synchronize(acf_stream stream);
 
+/* Device memory that this library holds without needing it goes back to the device: blocks of closed handles
+ * that it keeps for the next ones (at most 256 MB), and second copies of p and v that solvers and batches on
+ * the two-sweep scheme allocated for their runs and can do without (the next run that wants them allocates
+ * them anew). The library does so itself before one of its allocations fails; this call is for the other
+ * allocators of the process. It waits for the devices it frees memory on. Safe at any time, from any thread. */
+int acf_release_memory(void);
+
 /* Pinned host memory for fast state transfers. */
 int acf_host_alloc(size_t bytes, void **out);
 int acf_host_free(void *ptr);
