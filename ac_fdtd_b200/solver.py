@@ -177,6 +177,7 @@ class CudaAcousticFDTD:
         self._handle = handle
         self._finalizer = weakref.finalize(self, _free_native, handle.value)
         _native.check(self._lib.acf_set_graph(handle, int(steps_per_graph)), "acf_set_graph")
+        self.steps_per_graph = int(steps_per_graph)
 
         # Host snapshots: name -> ndarray, plus which are current and which were handed out.
         self._mirror: dict[int, np.ndarray] = {}
