@@ -4130,13 +4130,25 @@ int64_t run_resident(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStr
 // Whether a run of the two-sweep scheme takes its steps in pairs of fused steps, which end in the
 // room's own copy: (8 + 2R) elements moved per cell instead of (12 + 2R). In double precision the
 // fused step is the faster one at every size that is not held on chip (112^3 19.3 against 27.3 us,
-// 203 x 187 x 211 with every term 155 against 208). In single precision the sweeps are as fast or
-// faster while the state fits L2 (walls only: 160 x 161 x 163 34 against 38 us, 67 MB of state;
-// 176^3 47 against 42 us, 87 MB; 251 x 240 x 263 with every term 201 against 166), so from 0.6 of L2
-// on. It takes a second copy of p and v, so only where that is at most a sixteenth of the
+// 203 x 187 x 211 with every term 155 against 208). In single precision the sweeps are faster while the
+// state in place stays in L2 and its two copies do not, the more so the less a step computes, and longer where rows
+// are ragged: see one_sweep_l2. It takes a second copy of p and v, so only where that is at most a sixteenth of the
 // device memory free at the first such run, and in place otherwise.
-constexpr double kOneSweepL2 = 0.6;
 constexpr int64_t kOneSweepMinSteps = 8;
+
+// From which part of L2 the state in place takes fused steps, single precision. us per step of the sweeps and of the
+// fused step on both sides of each line: walls 156^3 32 and 33 (0.48), 172^3 42.4 and 41.6 (0.64), ragged 172^3 42.8
+// and 45.0 (0.64), 176^3 50 and 48 (0.70); no walls 172^3 31 and 34 (0.64), 176^3 38 and 35 (0.70), ragged 176^3 39 and
+// 42 (0.70), 180^3 44 and 41 (0.73); walls and air 140^3 37.7 and 38.5 (0.60), 144^3 42 and 40 (0.67), ragged 148^3
+// 45.2 and 46.0 (0.72), 156^3 52 and 52 (0.84); air alone 148^3 36 and 37 (0.71), 152^3 40 and 38 (0.79), ragged 168^3
+// 57 and 59 (1.07), 180^3 70 and 68 (1.28). With a layer the sweeps compute more: walls, air and layer 128^3 23 and
+// 26 (0.48), 140^3 48 and 40 (0.60), without walls ragged 140^3 and 164^3 7 and 10 % slower (0.61), 144^3 4 % faster.
+double one_sweep_l2(const RoomHost &h) {
+    const bool whole = h.nz % kVec == 0, air = h.n_relax > 0;
+    if (h.has_layer) return h.has_walls || whole ? 0.6 : 0.65;
+    if (h.has_walls) return air ? (whole ? 0.65 : 0.8) : (whole ? 0.6 : 0.68);
+    return air ? (whole ? 0.75 : 1.25) : (whole ? 0.67 : 0.72);
+}
 
 bool one_sweep_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
     if (b->one_sweep_state < 0 || n_steps < kOneSweepMinSteps || b->scheme != ACF_SCHEME_TWO_SWEEPS ||
@@ -4144,7 +4156,7 @@ bool one_sweep_ready(acf_batch *b, int64_t n_steps, cudaStream_t st) {
         return false;
     RoomHost &h = b->rooms[0];
     if (!fused_points(b)) return false;
-    if (b->precision == 4 && (double)b->room_block_bytes(0) < kOneSweepL2 * (double)b->l2_bytes) return false;
+    if (b->precision == 4 && (double)b->room_block_bytes(0) < one_sweep_l2(h) * (double)b->l2_bytes) return false;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
