@@ -3515,20 +3515,28 @@ const Room<T> *current_rooms(const acf_batch *b) {
     return (const Room<T> *)b->room_table + (b->rooms[0].cur ? b->rooms.size() : 0);
 }
 
-// Whether a batch on the fused scheme in single precision takes the two sweeps, in place in the current copy:
-// where the rooms in place stay in L2 and both their copies do not. us per step of the sweeps and of the fused step
-// (both copies in parts of L2), with air: 2 x 102^3 28 and 29 (0.73), 2 x 104^3 28 and 34 (0.82), 4 of 60 to 110 34
+// Whether a batch takes the two sweeps, in place in the current copy, instead of fused steps: where the rooms
+// in place stay in L2 and both their copies do not. us per step of the sweeps and of the fused step (both copies in
+// parts of L2), in single precision: with air 2 x 102^3 28 and 29 (0.73), 2 x 104^3 28 and 34 (0.82), 4 of 60 to 110 34
 // and 44 (0.98), 6 x 76^3 35 and 47 (0.96), 2 x 120^3 46 and 48 (1.24), 2 x 100^3 28.4 and 27.5 (0.70), 40 x 44^3 60
 // and 58 (1.29); without relaxation states 2 x 116^3 29 and 30 (0.79), 2 x 120^3 27 and 30 (0.90), 2 x 112^3 25.0 and
-// 24.8 (0.74), 2 x 122^3 42 and 37 (0.93). In double precision the fused step is the faster one throughout (2 x 92^3
-// 45 and 41, 2 x 128^3 128 and 93).
-bool batch_sweeps_faster(const acf_batch *b) {
-    if (b->precision == 8 || b->rooms.size() < 2) return false;
+// 24.8 (0.74), 2 x 122^3 42 and 37 (0.93), and with a layer, which costs the sweeps more, neither by over 7 %. In
+// double precision the fused step is the faster one throughout (2 x 92^3 45 and 41, 2 x 128^3 128 and 93).
+// Recorded steps also write the walls' history, the sweeps in one of their two passes; fused over sweeps:
+// walls 0.97 to 1.05 at 0.60, 1.26 at 0.70, 1.47 at 0.90, 0.95 to 1.02 at 0.93; a layer too 0.96 at 0.64, 1.05 at 0.71,
+// 1.25 at 0.90, 0.87 at 0.96; air 1.00 at 0.83, 1.06 at 0.86, 1.08 at 0.96, 1.04 at 1.16, 0.99 at 1.18; air and a layer
+// 0.86 to 1.02 throughout; in double precision without relaxation states 0.84 at 0.73, 1.09 at 0.89, 1.14 at 0.94, 0.98
+// to 1.02 at 1.02, with them 0.93 at most.
+bool batch_sweeps_faster(const acf_batch *b, bool recorded) {
+    if (b->rooms.size() < 2) return false;
     double bytes = 0.0;
-    for (size_t r = 0; r < b->rooms.size(); r++)
-        bytes += (double)(b->room_block_bytes((int)r) + (size_t)4 * b->rooms[r].field * b->elem());
+    for (size_t r = 0; r < b->rooms.size(); r++) bytes += (double)(b->room_block_bytes((int)r) + second_bytes(b, b->rooms[r]));
     const double both = bytes / (double)b->l2_bytes;
-    return b->n_relax > 0 ? both > 0.72 && both < 1.25 : both > 0.77 && both < 0.92;
+    const bool air = b->n_relax > 0, layer = b->any_layer;
+    auto between = [&](double low, double high) { return both > low && both < high; };
+    if (b->precision == 8) return recorded && !air && between(0.86, 0.945);
+    if (recorded) return air ? !layer && between(0.84, 1.17) : layer ? between(0.69, 0.92) : between(0.62, 0.925);
+    return air ? between(0.72, 1.25) : !layer && between(0.77, 0.92);
 }
 
 // Tiles in room order, then plane group, then (row, chunk) block: neighbouring tiles of one
@@ -4263,7 +4271,7 @@ int run_impl(acf_batch *b, int64_t n_steps, int64_t step_offset, cudaStream_t st
         n_steps -= last_in_place ? 1 : 0;
     }
     // The fused scheme where the sweeps are faster: in place in the current copy.
-    if (b->scheme == ACF_SCHEME_FUSED && (b->rooms.size() == 1 ? !fused_points(b) : batch_sweeps_faster(b)))
+    if (b->scheme == ACF_SCHEME_FUSED && (b->rooms.size() == 1 ? !fused_points(b) : batch_sweeps_faster(b, false)))
         b->scheme = ACF_SCHEME_TWO_SWEEPS;
 
     int64_t done = 0;
@@ -6029,7 +6037,7 @@ int batch_forward_record_impl(acf_batch *b, int64_t n_steps, int64_t step_offset
     // per step in single precision, 317 against 363 in double).
     int64_t most_points = 0;
     for (const RoomHost &h : b->rooms) most_points = std::max(most_points, points_of(h));
-    const bool one_sweep = !batch_sweeps_faster(b) && (b->scheme == ACF_SCHEME_FUSED || most_points <= kSomePoints) &&
+    const bool one_sweep = !batch_sweeps_faster(b, true) && (b->scheme == ACF_SCHEME_FUSED || most_points <= kSomePoints) &&
                            make_second_copies(b, st);
     if (one_sweep && b->room_table_dirty) {
         rc = upload_room_table<T>(b);
