@@ -94,26 +94,36 @@ def wall_gradients(walls, shape, grad_a, sound_speed, dt, dx):
     per-cell maps, from dL/da per shell slot."""
     cells = shell_face_gradients(shape, grad_a, sound_speed * dt / (2.0 * dx))
     if hasattr(walls, "patch_values"):
-        P = walls.patches
-        g = np.zeros((6, P, P))
-        for f, (axis, _) in enumerate(FACES):
-            b, c = [a for a in range(3) if a != axis]
-            ib = patch_index(shape[b], P)
-            ic = patch_index(shape[c], P)
-            np.add.at(g[f], (ib[:, None], ic[None, :]), cells[f])
-        return g, cells
+        return _patch_sums(walls.patches, shape, cells), cells
     return np.array([m.sum() for m in cells]), cells
+
+
+def _patch_sums(patches, shape, cells):
+    g = np.zeros((6, patches, patches))
+    for f, (axis, _) in enumerate(FACES):
+        b, c = [a for a in range(3) if a != axis]
+        ib = patch_index(shape[b], patches)
+        ic = patch_index(shape[c], patches)
+        np.add.at(g[f], (ib[:, None], ic[None, :]), cells[f])
+    return g
+
+
+#: Most patches along a wall that the device sums (``acf_adjoint_wall_gradients``).
+_DEVICE_PATCHES = 1024
 
 
 def _wall_gradients_of_run(call, walls, shape, sound_speed, dt, dx):
     """``wall_gradients`` of the run ``call(scale, patches, cells, sums)`` belongs to, mapped and
-    summed on the device."""
-    patches = int(walls.patches) if hasattr(walls, "patch_values") else 1
+    summed on the device (walls of more patches than that takes are summed here)."""
+    wanted = int(walls.patches) if hasattr(walls, "patch_values") else 1
+    patches = wanted if wanted <= _DEVICE_PATCHES else 1
     faces = [tuple(n for a, n in enumerate(shape) if a != axis) for axis, _ in FACES]
     ends = np.cumsum([b * c for b, c in faces])
     flat, sums = np.empty(int(ends[-1])), np.empty((6, patches, patches))
     call(sound_speed * dt / (2.0 * dx), patches, _as_double_pointer(flat), _as_double_pointer(sums))
     cells = [m.reshape(face) for m, face in zip(np.split(flat, ends[:-1]), faces)]
+    if patches != wanted:
+        return _patch_sums(wanted, shape, cells), cells
     return (sums if hasattr(walls, "patch_values") else sums.reshape(6)), cells
 
 
