@@ -317,21 +317,13 @@ pack_adjoint_batch(const BatchAdjointParams<T> b) {
     }
 }
 
-struct Shape {
-    dim3 grid, block;
-};
-
 template <typename T>
-Shape room_shape(const Room<T> &room, int planes, int block_threads) {
-    const int chunks = (room.nz + Pack<T>::W - 1) / Pack<T>::W;
-    int bx = 1;
-    while (bx < chunks && bx < 32) bx <<= 1;
-    const int by = std::max(1, std::min<int>(room.ny, std::min(block_threads, kPackThreads) / bx));
-    return {dim3((chunks + bx - 1) / bx, (room.ny + by - 1) / by, (room.nx + planes - 1) / planes), dim3(bx, by, 1)};
+ChunkShape room_shape(const Room<T> &room, int planes, int block_threads) {
+    return chunk_shape(room, planes, std::min(block_threads, kPackThreads));
 }
 
 template <typename T, bool L, bool W, int NR>
-void launch_one(const AdjointParams<T> &a, bool air, const Shape &q, cudaStream_t st) {
+void launch_one(const AdjointParams<T> &a, bool air, const ChunkShape &q, cudaStream_t st) {
     if constexpr (NR > 0) {
         if (air) {
             launch_after(pack_adjoint<T, L, W, NR, true>, q.grid, q.block, st, a);
@@ -341,12 +333,12 @@ void launch_one(const AdjointParams<T> &a, bool air, const Shape &q, cudaStream_
     launch_after(pack_adjoint<T, L, W, NR, false>, q.grid, q.block, st, a);
 }
 template <typename T, bool L, bool W, int NR>
-void launch_one(const BatchAdjointParams<T> &b, bool, const Shape &q, cudaStream_t st) {
+void launch_one(const BatchAdjointParams<T> &b, bool, const ChunkShape &q, cudaStream_t st) {
     launch_after(pack_adjoint_batch<T, L, W, NR>, q.grid, q.block, st, b);
 }
 
 template <typename T, bool L, bool W, typename P>
-void launch_relax(const P &p, int n_relax, bool air, const Shape &q, cudaStream_t st) {
+void launch_relax(const P &p, int n_relax, bool air, const ChunkShape &q, cudaStream_t st) {
     switch (n_relax) {
         case 0: launch_one<T, L, W, 0>(p, air, q, st); break;
         case 1: launch_one<T, L, W, 1>(p, air, q, st); break;
@@ -357,7 +349,7 @@ void launch_relax(const P &p, int n_relax, bool air, const Shape &q, cudaStream_
 }
 
 template <typename T, typename P>
-void launch_terms(const P &p, bool layer, bool walls, int n_relax, bool air, const Shape &q, cudaStream_t st) {
+void launch_terms(const P &p, bool layer, bool walls, int n_relax, bool air, const ChunkShape &q, cudaStream_t st) {
     if (layer) {
         if (walls) launch_relax<T, true, true>(p, n_relax, air, q, st);
         else launch_relax<T, true, false>(p, n_relax, air, q, st);
@@ -377,14 +369,14 @@ void launch_pack_adjoint(const AdjointParams<T> &a, bool layer, bool walls, int 
 
 template <typename T>
 int64_t pack_adjoint_blocks(const Room<T> &room, int planes, int block_threads) {
-    const Shape q = room_shape(room, planes, block_threads);
+    const ChunkShape q = room_shape(room, planes, block_threads);
     return (int64_t)q.grid.x * q.grid.y * q.grid.z;
 }
 
 template <typename T>
 void launch_pack_adjoint_batch(const BatchAdjointParams<T> &p, bool layer, bool walls, int n_relax, int ctas,
                                cudaStream_t st) {
-    launch_terms<T>(p, layer, walls, n_relax, false, Shape{dim3(ctas), dim3(kPackThreads)}, st);
+    launch_terms<T>(p, layer, walls, n_relax, false, ChunkShape{dim3(ctas), dim3(kPackThreads)}, st);
 }
 
 template void launch_pack_adjoint<float>(const AdjointParams<float> &, bool, bool, int, bool, int, cudaStream_t);

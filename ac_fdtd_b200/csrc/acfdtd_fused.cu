@@ -75,12 +75,7 @@ void launch_relax(const P &p, int n_relax, dim3 grid, dim3 block, bool early, cu
 template <typename T, typename P>
 void launch_room(const Room<T> &room, int planes, const P &p, bool layer, bool walls, int n_relax,
                  int block_threads, bool early, cudaStream_t st) {
-    const int chunks = (room.nz + Pack<T>::W - 1) / Pack<T>::W;
-    int bx = 1;
-    while (bx < chunks && bx < 32) bx <<= 1;
-    const int by = std::max(1, std::min<int>(room.ny, std::min(block_threads, 128) / bx));
-    const dim3 block(bx, by, 1);
-    const dim3 grid((chunks + bx - 1) / bx, (room.ny + by - 1) / by, (room.nx + planes - 1) / planes);
+    const auto [grid, block] = chunk_shape(room, planes, std::min(block_threads, kPackThreads));
     if (layer) {
         if (walls) launch_relax<true, true>(p, n_relax, grid, block, early, st);
         else launch_relax<true, false>(p, n_relax, grid, block, early, st);

@@ -142,6 +142,24 @@ __device__ __forceinline__ bool is_bad(double acc) { return acc != acc; }
 __device__ __forceinline__ float2 finite_start(float) { return dup2(0.f); }
 __device__ __forceinline__ double finite_start(double) { return 0.0; }
 
+// Blocks over a room's (row, chunk) columns, groups of `planes` x planes along z of the grid: up to 32 chunks of
+// a row, and rows, in at most `threads` threads. Rooms of so many rows that their blocks would exceed the
+// grid's 65535 take fewer chunks and more rows per block.
+struct ChunkShape {
+    dim3 grid, block;
+};
+
+template <typename T>
+ChunkShape chunk_shape(const Room<T> &room, int planes, int threads) {
+    const int chunks = (room.nz + Pack<T>::W - 1) / Pack<T>::W;
+    int bx = 1;
+    while (bx < chunks && bx < 32) bx <<= 1;
+    auto rows = [&]() { return threads / bx < 1 ? 1 : threads / bx < room.ny ? threads / bx : room.ny; };
+    while (bx > 1 && ((int64_t)room.ny + rows() - 1) / rows() > 65535) bx >>= 1;
+    const int by = rows();
+    return {dim3((chunks + bx - 1) / bx, (room.ny + by - 1) / by, (room.nx + planes - 1) / planes), dim3(bx, by, 1)};
+}
+
 }  // namespace acf
 
 #endif
