@@ -7,14 +7,17 @@ the caller's state is untouched. Results are cached per process, keyed by the sh
 dtype, which terms are active and whether runs may take many steps per launch, and optionally in a
 JSON file named by ``ACF_TUNE_CACHE``.
 
-Candidates are timed launch by launch. Runs of small rooms on the two-sweep and the fused scheme take
-many steps per launch instead (``acf_set_graph``), whatever the geometry, so those schemes count with
-the time of such a run: 64^3 in single precision 1.9 us per step, where the best launched step takes 8.6.
+Candidates are timed launch by launch, which finds each scheme's geometry. The schemes are then compared by runs
+as a program makes them, which are not the sum of their launches: runs of small rooms on the two-sweep and the
+fused scheme take many steps per launch (``acf_set_graph``; 64^3 in single precision 1.9 us per step, where the
+best launched step takes 8.6), and the fused steps of batches and of double precision start early, in the
+tail of the step before.
 """
 
 from __future__ import annotations
 
 import json
+import math
 import os
 import time
 from pathlib import Path
@@ -113,33 +116,33 @@ def _race(twin, candidates, apply, steps: int, repeats: int, passes: int) -> dic
     return timings
 
 
-#: Steps of the runs that rooms held on chip are timed by: their launch and its wait count for 1 % at 2 us a step.
-HELD_STEPS = 1024
+def _run_ms(twin, steps: int = 64, least_ms: float = 5.0) -> float:
+    """ms/step of ``twin``'s runs as a program makes them: replayed from graphs, launched early into the
+    step before, or held on chip. Long enough that the wait at their end counts for little."""
+
+    def timed(n: int) -> float:
+        start = time.perf_counter()
+        twin.run(n)
+        twin.synchronize()
+        return 1e3 * (time.perf_counter() - start) / n
+
+    timed(steps)                                   # graphs and buffers
+    steps *= max(1, min(32, math.ceil(least_ms / max(steps * timed(steps), 1e-3))))
+    return min(timed(steps) for _ in range(3))
 
 
-def _held_times(twin, schemes) -> dict:
-    """ms/step of a run as ``twin`` makes it, for the schemes that take many steps per launch."""
-    times = {}
-    for scheme in schemes:
-        if scheme not in ("two_sweeps", "fused"):
-            continue
-        try:
-            twin.set_scheme(scheme)
-        except RuntimeError:
-            continue
-        before = twin.launch_count()
-        twin.run(16)
-        if twin.launch_count() - before >= 16:
-            continue
-        best = float("inf")
-        for _ in range(3):
-            twin.synchronize()
-            start = time.perf_counter()
-            twin.run(HELD_STEPS)
-            twin.synchronize()
-            best = min(best, 1e3 * (time.perf_counter() - start) / HELD_STEPS)
-        times[scheme] = best
-    return times
+def _final(twin, launched: dict, apply) -> tuple:
+    """The fastest of each scheme's best candidate, by runs; and all timings, theirs by runs."""
+    best: dict = {}
+    for candidate, ms in launched.items():
+        if candidate[0] not in best or ms < launched[best[candidate[0]]]:
+            best[candidate[0]] = candidate
+    timings = dict(launched)
+    if len(best) > 1:
+        for candidate in best.values():
+            apply(twin, candidate)
+            timings[candidate] = _run_ms(twin)
+    return min(best.values(), key=timings.get), timings
 
 
 def tune(solver, candidates=CANDIDATES, steps: int = 12, repeats: int = 2, schemes=SCHEMES,
@@ -155,13 +158,9 @@ def tune(solver, candidates=CANDIDATES, steps: int = 12, repeats: int = 2, schem
     try:
         launched = _race(twin, _candidates(schemes, candidates, staged_candidates), _apply, steps,
                          repeats, passes)
-        held = _held_times(twin, schemes)
+        return _final(twin, launched, _apply)
     finally:
         twin.close()
-    timings = {c: held.get(c[0], ms) for c, ms in launched.items()}
-    # runs too short to be held take the launched step: the fastest of those that tie
-    winner = min(timings, key=lambda c: (timings[c], launched[c]))
-    return winner, timings
 
 
 def apply_tuned(solver, candidates=CANDIDATES, schemes=SCHEMES,
@@ -192,14 +191,13 @@ def tune_batch(batch, candidates=BATCH_CANDIDATES, steps: int = 12, repeats: int
     """Time each batch geometry on a scratch twin batch; return (best, {candidate: ms/step})."""
     from .batch import RoomBatch
 
-    twin = RoomBatch(batch.specs, dtype=batch.dtype, steps_per_graph=0)
+    twin = RoomBatch(batch.specs, dtype=batch.dtype, steps_per_graph=batch.steps_per_graph)
     try:
         for r in range(len(twin)):
             twin.set_field(r, 0, np.random.default_rng(r).standard_normal(twin.shapes[r]) * 1e-3)
-        timings = _race(twin, candidates, _apply_batch, steps, repeats, passes)
+        return _final(twin, _race(twin, candidates, _apply_batch, steps, repeats, passes), _apply_batch)
     finally:
         twin.close()
-    return min(timings, key=timings.get), timings
 
 
 def apply_tuned_batch(batch, candidates=BATCH_CANDIDATES):

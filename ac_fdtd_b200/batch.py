@@ -92,6 +92,7 @@ class RoomBatch:
         self._stream = ctypes.c_void_p(int(stream))
         _native.check(self._lib.acf_batch_set_graph(handle, int(steps_per_graph)),
                       "acf_batch_set_graph")
+        self.steps_per_graph = int(steps_per_graph)
         self.step_index = 0
         self._sources = [[] for _ in rooms]
         self._receivers = [[] for _ in rooms]
