@@ -22,6 +22,10 @@ __device__ __forceinline__ void pack_column(const FusedParams<T> &f, int i_begin
                                             int64_t step, const History<T> *hist = nullptr) {
     using P = Pack<T>;
     constexpr int W = P::W;
+    // With a layer in single precision the relaxation states are loaded after the faces: held through the damping of
+    // the faces they do not fit the 96 registers of 20 warps per SM (136 bytes spilled, so 72; 8 rooms of 96 to 180
+    // with air and a layer 331 us per step, so 295; at 128 registers and 16 warps 319).
+    constexpr bool STATES_LATE = LAYER && sizeof(T) == 4 && !REC;
     const Room<T> &s = f.room;
     const int k0 = c * W, real = min(W, s.nz - k0);
     const bool tail = real < W;
@@ -45,20 +49,29 @@ __device__ __forceinline__ void pack_column(const FusedParams<T> &f, int i_begin
         damp_y = fy_c != T(1) || fy_l != T(1) || fy_h != T(1);
 #pragma unroll
         for (int e = 0; e <= W; e++) {
-            damp_z = damp_z || __ldg(s.face[2] + min(k0 + e, s.nz)) != T(1);
-            if (e < W) damp_z = damp_z || __ldg(s.cell[2] + min(k0 + e, s.nz - 1)) != T(1);
+            const T face = __ldg(s.face[2] + min(k0 + e, s.nz));
+            damp_z = damp_z || face != T(1);
+            if (e < W) {
+                const T cell = __ldg(s.cell[2] + min(k0 + e, s.nz - 1));
+                damp_z = damp_z || cell != T(1);
+            }
         }
     }
     // z factors at cells and at faces, read where used (they stay in L1)
-    auto z_times = [&](const P &v, const T *profile, int last) {
+    auto z_cells = [&](const P &v) {
         T x[W];
         unpack(v, x);
 #pragma unroll
-        for (int e = 0; e < W; e++) x[e] = x[e] * __ldg(profile + min(k0 + e, last));
+        for (int e = 0; e < W; e++) x[e] = x[e] * __ldg(s.cell[2] + min(k0 + e, s.nz - 1));
         return repack(x);
     };
-    auto z_cells = [&](const P &v) { return z_times(v, s.cell[2], s.nz - 1); };
-    auto z_faces = [&](const P &v) { return z_times(v, s.face[2], s.nz); };
+    auto z_faces = [&](const P &v) {
+        T x[W];
+        unpack(v, x);
+#pragma unroll
+        for (int e = 0; e < W; e++) x[e] = x[e] * __ldg(s.face[2] + min(k0 + e, s.nz));
+        return repack(x);
+    };
     auto moved = [&](const P &v, const P &high, const P &low) { return psub(v, pmul(psub(high, low), cv)); };
 
     // Carried from plane to plane: p(i) and the updated vx on face i.
@@ -90,7 +103,7 @@ __device__ __forceinline__ void pack_column(const FusedParams<T> &f, int i_begin
 #pragma unroll
             for (int r = 0; r < NR; r++) prefetch_l2(s.psi + r * s.field + next);
         }
-        // ---- loads, all before the first store
+        // ---- loads, before the first store
         P ph = pload(s.p + base + (inner ? s.plane : 0));
         const P py_l = pload(s.p + base + y_lo), py_h = pload(s.p + base + y_hi);
         P xh = pload(s.vx + base + s.plane), yl = pload(s.vy + base), yh = pload(s.vy + base + s.pz);
@@ -98,8 +111,11 @@ __device__ __forceinline__ void pack_column(const FusedParams<T> &f, int i_begin
         const T pz_l = s.p[base + z_lo], pz_h = s.p[base + z_hi];
         T za = k0 + W <= s.nz ? s.vz[base + W] : T(0);
         P S[NR > 0 ? NR : 1];
+        auto load_states = [&]() {
 #pragma unroll
-        for (int r = 0; r < NR; r++) S[r] = pload(s.psi + r * s.field + base);
+            for (int r = 0; r < NR; r++) S[r] = pload(s.psi + r * s.field + base);
+        };
+        if (!STATES_LATE) load_states();
 
         // ---- the faces
         if (tail) ph = mirrored(ph, real);
@@ -134,6 +150,7 @@ __device__ __forceinline__ void pack_column(const FusedParams<T> &f, int i_begin
                 za = za * __ldg(s.face[2] + min(k0 + W, s.nz));
             }
         }
+        if (STATES_LATE) load_states();
         // ---- the cells
         P d = psub(xh, xl);
         d = padd(d, psub(yh, yl));
