@@ -4,12 +4,14 @@
 // read and written every step, and below 10^6 cells a step costs its launches and their latency,
 // not its bytes: in two launches per step 64^3 took 10.0 us (single precision) and 13.0 us (double),
 // and 32^3 no less. Here one cooperative launch holds the room and takes every step; a step then
-// costs one exchange between neighbour CTAs and its arithmetic. Measured per step, walls only:
-// 32^3 1.3 us (from 10.1, single) and 1.3 us (from 12.6, double), 64^3 1.8 and 2.7 us, 80^3 2.8 and
-// 5.3 us (from 10.3 and 12.6), 96^3 4.9 and 12.3 us (from 10.8 and 15.8), 128^3 11.6 us (from 14.2,
-// single). What bounds it: up to 64^3 the exchange -- a store seen by another SM takes 500
-// cycles on the same die and 900 on the other, so about 1500 with the poll and the barrier of
-// 2300 to 3300 a step -- and above it the instructions, at 4 warps per scheduler.
+// costs one exchange between neighbour CTAs and its arithmetic. Measured per step, walls only, against the
+// two sweeps: 32^3 1.3 us (from 10.1, single) and 1.3 us (from 12.6, double), 64^3 1.9 and 2.7 us, 80^3 2.8
+// and 5.3 us (from 10.8 and 13.1), 96^3 5.2 us (from 11.6, single), 128^3 12.1 us (from 14.8, single);
+// against the fused step 64^3 8.6 and 10.6, 80^3 8.2 and 10.8, 96^3 8.9 (single). Larger rooms are not always
+// faster on chip: see resident_faster. What bounds it: up to 64^3 the exchange -- a store seen by another
+// SM takes 500 cycles on the same die and 900 on the other, so about 1500 with the poll and the barrier of
+// 2300 to 3300 a step; its warps wait at the barrier most -- and above it latency: 3 or 4 warps per scheduler, whose
+// instructions wait for one another and for shared memory, issue in a third of the cycles.
 //
 // One CTA per SM owns a brick of the room, a thread K consecutive x planes of one (row, 16-byte
 // chunk) column: velocities in the thread's registers, p in shared memory. Only p crosses bricks:
@@ -893,7 +895,11 @@ const void *resident_kernel(int planes, int n_relax, bool layer) {
 }  // namespace
 
 // Among all bricks that fit, the one with the least work per step: warps x planes of arithmetic,
-// plus the rim its threads receive.
+// plus the rim its threads receive. The weights are rough, and only rank the bricks of one room: three states held
+// cost 10 to 20 % of a step (64^3 1.95 and 2.15 us, 96^3 5.2 and 5.9), one left in L2 more than all the held ones
+// (112^3, two of three held, 8.7 and 13.9). The two-barrier form takes 1.0 to 1.4 times as long per chunk (96^3, 4
+// planes of 384 threads, 5.2 and with air 5.9; 104^3, 6 of 352, 8.4 and 11.5); weighted twice, it is left to the rooms
+// that the other does not fit. Whether the plan beats the step it replaces is resident_faster's question.
 template <typename T>
 ResidentPlan resident_plan(int nx, int ny, int nz, int n_relax, bool layer, int sms, size_t smem_limit) {
     constexpr int W = Pack<T>::W;

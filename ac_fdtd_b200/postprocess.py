@@ -7,8 +7,8 @@ decay, T20/T30, EDT, clarity). Here the same steps run where the recordings alre
 * ``deconvolve`` -- real-to-complex FFT of the recordings and the excitation (cuFFT through
   ``torch.fft``: a library FFT, off the leapfrog's path), the regularised spectral division
   and band limit in this library's kernel (``acf_spectral_divide``), inverse FFT;
-* ``schroeder_decay`` -- the backward integral of the squared signal as a CTA-wide scan
-  (``acf_schroeder_decay``);
+* ``schroeder_decay`` -- the backward integral of the squared signal as a scan by one CTA per signal, or a cluster
+  of CTAs for long ones (``acf_schroeder_decay``);
 * ``reverberation_time`` / ``early_decay_time`` -- the least-squares slope between two levels of
   the decay curve (``acf_decay_fit``);
 * ``clarity`` -- the early-to-late energy split (``acf_clarity``).

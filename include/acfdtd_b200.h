@@ -149,10 +149,13 @@ int acf_pressure_only_energy_terms(acf_solver *solver, double terms[2], acf_stre
 /* How a single room advances: two sweeps per step over one copy of the state, or one fused
  * sweep that reads the current p and v and writes the next ones to a second copy (4 more
  * fields of memory, (8 + 2R) instead of (12 + 2R) elements moved per cell). Both give
- * bit-identical results. The adjoint's recorded runs use the two sweeps. Runs of 8 steps or
- * more on the two-sweep scheme may take pairs of fused steps inside, ending in the one copy the
- * caller sees, where that is faster and a second copy takes at most a sixteenth of the free device
- * memory (neither when profiling or launching step by step, see acf_set_graph, nor in a capture).
+ * bit-identical results. Runs of 8 steps or more on the two-sweep scheme may take pairs of fused steps
+ * inside, ending in the one copy the caller sees, where that is faster and a second copy takes at most a
+ * sixteenth of the free device memory (neither when profiling or launching step by step, see acf_set_graph,
+ * nor in a capture); recorded runs (acf_forward_record) too, without that limit. The second copy
+ * stays until the handle closes or something else needs the memory (acf_release_memory). In the other
+ * direction, runs on the fused scheme take the two sweeps, in place in the copy that is current, where
+ * those are faster.
  * ACF_SCHEME_FUSED_STAGED is the fused sweep with each CTA's share of every x plane streamed
  * into a shared-memory ring by bulk copies (see acf_set_staging); same memory, same results.
  * No counterpart in the reference (its C loop runs the two sweeps, acfdtd.c:355-376). */
