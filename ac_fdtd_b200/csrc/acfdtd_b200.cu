@@ -3601,8 +3601,10 @@ int pack_planes(const acf_batch *b) {
 int build_tiles(acf_batch *b) {
     int rc = upload_tiles(b, kVec, b->block_threads, b->planes, &b->tiles, &b->n_tiles, &b->batch_ctas);
     if (rc) return rc;
-    return upload_tiles(b, 16 / (int)b->elem(), std::min(b->block_threads, kPackThreads), pack_planes(b),
-                        &b->pack_tiles, &b->n_pack_tiles, &b->pack_ctas);
+    // its blocks have kPackThreads threads whatever the sweeps' have: smaller tiles would leave the rest idle
+    // (4 x 192^3 with walls 215 against 181 us per step with tiles of 64)
+    return upload_tiles(b, 16 / (int)b->elem(), kPackThreads, pack_planes(b), &b->pack_tiles, &b->n_pack_tiles,
+                        &b->pack_ctas);
 }
 
 struct LaunchShape {
