@@ -56,3 +56,9 @@ def test_a_single_scheme_is_not_timed_again():
     launched = {c: ms for c, ms in twin.launched.items() if c[0] == "fused"}
     winner, timings = autotune._final(twin, launched, lambda *_: pytest.fail("applied again"))
     assert winner == ("fused", 128, 8, 0) and timings == launched
+
+
+def test_batch_candidates_hold_the_planes_that_untuned_batches_take():
+    """An untuned batch takes 4 to 8 planes per tile of the fused step; tuned, it has to find one at least as good."""
+    planes = {c[2] for c in autotune.BATCH_CANDIDATES if c[0] == "fused" and c[3] == 0}
+    assert {4, 5, 6, 8} <= planes
