@@ -4,6 +4,7 @@ allocation that would fail otherwise, or to a request; the runs after that have 
 
 from __future__ import annotations
 
+import gc
 import threading
 
 import numpy as np
@@ -23,6 +24,7 @@ def _grid(nx, ny, nz):
 
 
 def _free(torch):
+    gc.collect()                     # solvers that other tests left to the collector
     torch.cuda.synchronize()
     return torch.cuda.mem_get_info()[0]
 
