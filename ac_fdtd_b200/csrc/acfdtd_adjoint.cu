@@ -322,6 +322,20 @@ ChunkShape room_shape(const Room<T> &room, int planes, int block_threads) {
     return chunk_shape(room, planes, std::min(block_threads, kPackThreads));
 }
 
+// Planes per block: fewer than `planes` while the blocks would leave SMs idle, since a small room's step is
+// the chain of its planes' loads and wall terms (20 x 21 x 23 with air in single precision, 10 blocks of four planes:
+// 18.9 us per step of the gradient's backward run with all its host work, 16.8 with the step of two elements per thread
+// before it, 10.8 so).
+template <typename T>
+int room_planes(const Room<T> &room, int planes, int block_threads) {
+    constexpr int kSms = 148;
+    for (; planes > 1; planes = (planes + 1) / 2) {
+        const ChunkShape q = room_shape(room, planes, block_threads);
+        if ((int64_t)q.grid.x * q.grid.y * q.grid.z >= kSms) break;
+    }
+    return planes;
+}
+
 template <typename T, bool L, bool W, int NR>
 void launch_one(const AdjointParams<T> &a, bool air, const ChunkShape &q, cudaStream_t st) {
     if constexpr (NR > 0) {
@@ -364,12 +378,14 @@ void launch_terms(const P &p, bool layer, bool walls, int n_relax, bool air, con
 template <typename T>
 void launch_pack_adjoint(const AdjointParams<T> &a, bool layer, bool walls, int n_relax, bool air, int block_threads,
                          cudaStream_t st) {
-    launch_terms<T>(a, layer, walls, n_relax, air, room_shape(a.room, a.planes, block_threads), st);
+    AdjointParams<T> q = a;
+    q.planes = room_planes(a.room, a.planes, block_threads);
+    launch_terms<T>(q, layer, walls, n_relax, air, room_shape(a.room, q.planes, block_threads), st);
 }
 
 template <typename T>
 int64_t pack_adjoint_blocks(const Room<T> &room, int planes, int block_threads) {
-    const ChunkShape q = room_shape(room, planes, block_threads);
+    const ChunkShape q = room_shape(room, room_planes(room, planes, block_threads), block_threads);
     return (int64_t)q.grid.x * q.grid.y * q.grid.z;
 }
 
